@@ -20,6 +20,7 @@
 #include "quartic.h"
 #include "solvers_host.h"
 #include "trajectory.h"
+#include "trajectory_tile.h"
 
 namespace rcmps {
 
@@ -316,6 +317,7 @@ int rcmps_context_create(int device, rcmps_context** out) {
   }
   ctx->stream = ctx->slot[0].stream;
   if (e == cudaSuccess) e = trajectory_set_tables();
+  if (e == cudaSuccess) e = tile_trajectory_init();
   if (e == cudaSuccess) e = quartic_init();
   if (e != cudaSuccess) {
     rcmps_context_destroy(ctx);

@@ -182,6 +182,47 @@ cudaError_t launch_z2_check(const double* R, const double* K, const double* rho,
   return cudaGetLastError();
 }
 
+// One CTA per state: whether rho is Hermitian to rounding. The comparison is false for a NaN.
+__global__ void hermitian_check_kernel(const double2* __restrict__ rho, int dp, long long stride,
+                                       int* __restrict__ flags, long long flag_stride) {
+  const double2* p = rho + (long long)blockIdx.x * stride;
+  __shared__ double red[2][32];
+  double top = 0.0, off = 0.0;
+  for (int e = threadIdx.x; e < dp * dp; e += blockDim.x) {
+    const int i = e / dp, j = e % dp;
+    const double2 a = p[e], b = p[j * dp + i];
+    const double d = fmax(fabs(a.x - b.x), fabs(a.y + b.y));
+    top = fmax(top, fmax(fabs(a.x), fabs(a.y)));
+    off = d <= off ? off : d;   // keeps a NaN
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    const double d = __shfl_xor_sync(0xffffffffu, off, o);
+    off = d <= off ? off : d;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = top;
+    red[1][threadIdx.x >> 5] = off;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
+      top = fmax(top, red[0][w]);
+      off = red[1][w] <= off ? off : red[1][w];
+    }
+    flags[blockIdx.x * flag_stride] = off <= 8.0 * 2.220446049250313e-16 * top ? 1 : 0;
+  }
+}
+
+cudaError_t launch_hermitian_check(const double* rho, int dp, long long in_stride, int nstates, int* flags,
+                                   long long flag_stride, cudaStream_t stream) {
+  if (nstates == 0) return cudaSuccess;
+  note_launch();
+  hermitian_check_kernel<<<nstates, 256, 0, stream>>>(reinterpret_cast<const double2*>(rho), dp, in_stride, flags,
+                                                      flag_stride);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_pad(const double* src, const long long* d_src_off, const int* d_dims, double* dst, int dp,
                        long long stride, int nstates, cudaStream_t stream) {
   if (nstates == 0) return cudaSuccess;

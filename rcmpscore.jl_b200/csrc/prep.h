@@ -33,6 +33,9 @@ cudaError_t launch_endpoint_trace(const double2* samples, long long stride, long
 cudaError_t launch_z2_check(const double* R, const double* K, const double* rho, const int* d_dims, int dp,
                             long long in_stride, int nstates, int mode, int* z2_flags, long long flag_stride,
                             cudaStream_t stream);
+// flags[i] = 1 where rho is Hermitian to rounding: |rho_ij - conj(rho_ji)| <= 8 eps max|rho| entrywise.
+cudaError_t launch_hermitian_check(const double* rho, int dp, long long in_stride, int nstates, int* flags,
+                                   long long flag_stride, cudaStream_t stream);
 cudaError_t launch_prepare(const double* R, const double* K, const double* rho, double* ops, int dp,
                            long long in_stride, long long ops_stride, int nstates, cudaStream_t stream);
 }  // namespace rcmps

@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 #include "../../include/rcmps_b200.h"
@@ -14,6 +15,7 @@
 #include "pullback.h"
 #include "quartic.h"
 #include "trajectory.h"
+#include "trajectory_tile.h"
 
 namespace rcmps {
 
@@ -33,8 +35,9 @@ struct Layout {
 constexpr int kNodesPerBlock = 32;
 
 // Per-system sizes: channels of a stage vector, operator matrices, stage vectors of the
-// trajectory workspace (y, prop, k[16], z[2], P, and L for the all-ODE route), pullback
-// scratch, partial and finalize matrices per state.
+// trajectory workspace (k[18], the last two of them y and prop, z[2], P, and L for the all-ODE
+// route; the quartic system's tile kernel has z[3] and P[16]), pullback scratch, partial and
+// finalize matrices per state.
 struct SysSizes {
   int nch, nops, nwork;
   size_t wscr, part, fin;   // in dp x dp matrices per state
@@ -44,7 +47,7 @@ SysSizes sys_sizes(int system, int dp, int nblk) {
   z.nch = trajectory_channels(system);
   if (system == 0) {
     z.nops = kOps;
-    z.nwork = 21;
+    z.nwork = 37;
     z.wscr = (size_t)nblk * pullback_row_blocks(dp) * 3;
     z.part = (size_t)nblk * 4;
     z.fin = 8;
@@ -76,7 +79,7 @@ size_t state_bytes(int system, int dp, int npoints, int nodes, bool split = fals
   b += (size_t)z.nwork * z.nch * mat;           // trajectory workspace
   b += (size_t)npoints * z.nch * mat;           // samples
   b += (z.wscr + z.part + z.fin + 2) * mat;     // pullback scratch, partials, finalize, cov/env
-  b += 1024;                                    // small per-state records
+  b += 1024 + align256(tile_sync_bytes());      // small per-state records
   if (split) b += split_state_bytes();          // BF16 slices of the constant operands
   return b;
 }
@@ -219,6 +222,7 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
       const size_t o_flag = L.add(n * sizeof(int));
       const size_t o_states = L.add(n * sizeof(TrajState));
       const size_t o_tstats = L.add(n * sizeof(TrajStats));
+      const size_t o_sync = L.add(n * tile_sync_bytes());
       const size_t o_in = L.add(3 * n * mat * 16);
       const size_t o_ops = L.add((size_t)n * zs.nops * mat * 16);
       const size_t o_work = L.add((size_t)n * zs.nwork * NCH * mat * 16);
@@ -247,7 +251,7 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
       const size_t h_o_tstats = H.add(n * sizeof(TrajStats));
       const size_t h_o_flag = H.add(n * sizeof(int));
       const size_t h_o_vals = H.add(n * 8);
-      const size_t h_o_z2 = H.add(n * sizeof(int));
+      const size_t h_o_z2 = H.add(2 * n * sizeof(int));
       if (pinned_reserve(SL, H.total) != cudaSuccess) return fail(ctx, RCMPS_CUDA_ERROR, "pinned host buffer");
       char* h = static_cast<char*>(SL.pinned);
       int* h_dims = reinterpret_cast<int*>(h + h_o_dims);
@@ -290,11 +294,11 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
           t.Ch = ops + kCh * mat;
         }
         double2* w = d_work + (size_t)i * zs.nwork * vec;
-        t.y = w;
-        t.prop = w + vec;
-        t.k = w + 2 * vec;
+        t.k = w;
+        t.y = w + 16 * vec;
+        t.prop = w + 17 * vec;
         t.z = w + 18 * vec;
-        t.P = w + 20 * vec;
+        t.P = w + (system == 0 ? 21 : 20) * vec;
         t.L = system == 1 ? w + 21 * vec : nullptr;
         t.samples = d_samp + (size_t)i * npoints * vec;
         t.stats = reinterpret_cast<TrajStats*>(base + o_tstats) + i;
@@ -336,23 +340,34 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
         e = launch_z2_check(dR, dK, dP, (int*)P(o_dims), dp, in_stride, n, S.symmetry,
                             reinterpret_cast<int*>(base + o_states + offsetof(TrajState, z2)),
                             (long long)(sizeof(TrajState) / sizeof(int)), stream);
-      if (e == cudaSuccess && system == 0 && S.symmetry == 1) {
-        // the strict route fails before any integration, as the reference raises in the
-        // constructor of its packed system
+      // The tile kernel takes the states with a Hermitian density unless the caller asked for the
+      // split products or for a row-block layout; the row-block kernel takes the others.
+      const bool tile_route = system == 0 && !split && S.trajectory_groups == 0;
+      const int teams = tile_route ? tile_trajectory_teams(dp, n) : 0;
+      if (e == cudaSuccess && teams)
+        e = launch_hermitian_check(dP, dp, in_stride, n, reinterpret_cast<int*>(base + o_states + offsetof(TrajState, herm)),
+                                   (long long)(sizeof(TrajState) / sizeof(int)), stream);
+      int nherm = 0;
+      if (e == cudaSuccess && (teams || (system == 0 && S.symmetry == 1))) {
+        // both flags of every state (z2, herm), read back before the trajectories: the strict packed
+        // route fails before any integration, as the reference raises in the constructor of its
+        // packed system, and the second kernel is launched only for states that need it
+        static_assert(offsetof(TrajState, herm) == offsetof(TrajState, z2) + sizeof(int), "adjacent flags");
         int* h_z2 = reinterpret_cast<int*>(h + h_o_z2);
-        e = cudaMemcpy2DAsync(h_z2, sizeof(int), base + o_states + offsetof(TrajState, z2), sizeof(TrajState),
-                              sizeof(int), n, cudaMemcpyDeviceToHost, stream);
+        e = cudaMemcpy2DAsync(h_z2, 2 * sizeof(int), base + o_states + offsetof(TrajState, z2), sizeof(TrajState),
+                              2 * sizeof(int), n, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        if (e == cudaSuccess)
-          for (int i = 0; i < n; ++i)
-            if (h_z2[i] < 0) {
-              job.stats[idx[i]].status = RCMPS_INVALID_ARGUMENT;
-              job.stats[idx[i]].failed_component = 1;
-              return fail(ctx, RCMPS_INVALID_ARGUMENT,
-                          "state " + std::to_string(idx[i]) +
-                              ": the packed Z2 route requires an even D and the exact block structure "
-                              "(R odd, K and rho even, rho Hermitian to 1e-13); no projection is performed");
-            }
+        for (int i = 0; e == cudaSuccess && i < n; ++i) {
+          nherm += h_z2[2 * i + 1];
+          if (S.symmetry == 1 && h_z2[2 * i] < 0) {
+            job.stats[idx[i]].status = RCMPS_INVALID_ARGUMENT;
+            job.stats[idx[i]].failed_component = 1;
+            return fail(ctx, RCMPS_INVALID_ARGUMENT,
+                        "state " + std::to_string(idx[i]) +
+                            ": the packed Z2 route requires an even D and the exact block structure "
+                            "(R odd, K and rho even, rho Hermitian to 1e-13); no projection is performed");
+          }
+        }
       }
       if (e == cudaSuccess)
         e = node_weights_launch((double*)P(o_points), (double*)P(o_weights), nodes, (double*)P(o_wj), stream);
@@ -360,13 +375,24 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
       tc.endpoint = points.back();
       tc.initial_h = S.initial_step;
       tc.max_ns = (unsigned long long)(S.max_device_seconds * 1e9);
-      tc.groups = trajectory_groups(system, dp, n, S.trajectory_groups, split ? 1 : 0);
-      ctx->traj_groups[system][dp_index(dp)] = tc.groups;
-      if (!split) tc.ring = ring_for_launch(ctx, system, dp, group_level(tc.groups));
+      const bool rows = nherm < n;   // states for the row-block kernel
+      if (rows) tc.groups = trajectory_groups(system, dp, n, S.trajectory_groups, split ? 1 : 0);
+      ctx->traj_groups[system][dp_index(dp)] = rows ? tc.groups : std::min(teams, 4);
+      if (rows && !split) tc.ring = ring_for_launch(ctx, system, dp, group_level(tc.groups));
       if (e == cudaSuccess) e = cudaEventRecord(e0, stream);
-      if (e == cudaSuccess)
+      // Teams of one state wait for one another, so only one launch of several teams is in flight on a
+      // device: two that share the SMs could each hold part of them and wait for the rest. Held to the
+      // end of this sub-batch; other contexts' launches of one team per state go ahead.
+      std::unique_lock<std::mutex> alone;
+      if (nherm && teams > 1) alone = std::unique_lock<std::mutex>(tile_trajectory_mutex(ctx->device));
+      if (e == cudaSuccess && nherm)
+        e = tile_trajectory_launch(dp, (TrajState*)P(o_states), n, (double*)P(o_points), npoints, tc, P(o_sync), teams,
+                                   S.symmetry != 0, stream);
+      if (e == cudaSuccess && rows) {
+        tc.skip_hermitian = nherm > 0 ? 1 : 0;
         e = trajectory_launch(system, dp, (TrajState*)P(o_states), n, (double*)P(o_points), npoints, tc, stream,
                               split ? 1 : 0);
+      }
       if (e == cudaSuccess) e = cudaEventRecord(e1, stream);
       if (e != cudaSuccess) return fail(ctx, RCMPS_CUDA_ERROR, std::string("trajectory launch: ") + cudaGetErrorString(e));
       // copy the trajectory values into a plain array for the finalize step
@@ -461,7 +487,7 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
       float ms = 0.f;
       cudaEventElapsedTime(&ms, e0, e1);
       traj_ms += ms;
-      if (!split) {
+      if (!split && !nherm) {
         long long longest = 0;
         for (int i = 0; i < n; ++i)
           longest = std::max(longest, 1 + 12 * h_tstats[i].attempts + 3 * h_tstats[i].dense_steps);

@@ -33,44 +33,11 @@
 #include <cstdio>
 #include <cstring>
 #include "common.cuh"
-#include "dop853_tables.h"
+#include "dop853_device.cuh"
 #include "split.cuh"
-#include "source_table.h"
 #include "trajectory.h"
 
 namespace rcmps {
-
-__constant__ double c_dop_a[256];
-__constant__ double c_dop_b[16];
-__constant__ double c_dop_c[16];
-__constant__ double c_dop_e5[16];
-__constant__ double c_dop_e3[16];
-__constant__ double c_dop_d[64];
-__constant__ double c_source[RCMPS_SOURCE_SEGMENTS * (RCMPS_SOURCE_DEGREE + 1)];
-
-// 2|t| J(t^2) from the piecewise Chebyshev table (Clenshaw); |t| <= sqrt(40).
-__device__ double source_value(double t) {
-  const double a = fabs(t);
-  const double width = RCMPS_SOURCE_AMAX / RCMPS_SOURCE_SEGMENTS;
-  int seg = (int)(a / width);
-  if (seg > RCMPS_SOURCE_SEGMENTS - 1) seg = RCMPS_SOURCE_SEGMENTS - 1;
-  const double z = 2.0 * (a - seg * width) / width - 1.0;
-  const double* c = c_source + seg * (RCMPS_SOURCE_DEGREE + 1);
-  double b1 = 0.0, b2 = 0.0;
-  for (int j = RCMPS_SOURCE_DEGREE; j > 0; --j) {
-    const double b0 = 2.0 * z * b1 - b2 + c[j];
-    b2 = b1;
-    b1 = b0;
-  }
-  return z * b1 - b2 + c[0];
-}
-
-// The next double above t (nextafter(t, +inf)) for finite t.
-__device__ __forceinline__ double next_up(double t) {
-  if (t == 0.0) return 4.9406564584124654e-324;
-  const long long b = __double_as_longlong(t);
-  return __longlong_as_double(t > 0.0 ? b + 1 : b - 1);
-}
 
 // Channel tables of the two systems (filled by trajectory_set_tables).
 //   g1: the G1 products in order: channel and panel kind (0 [Q;R] rows, 1 [Q^dag;R^dag] rows,
@@ -660,6 +627,7 @@ trajectory_kernel(const TrajState* __restrict__ states, const double* __restrict
   const uint32_t rank = cluster_rank();
   const int sidx = (int)cluster_id_x();
   const TrajState* st = states + sidx;
+  if (SYS == kSysQuartic && ctl_in.skip_hermitian && st->herm) return;   // the whole cluster
   // cluster of G x CG CTAs: rows 16 (rank % G) .. + 15 of the channel group rank / G
   const uint32_t nrank = cluster_size();
   const int ngroups = (int)nrank / GE::G;
@@ -1407,12 +1375,7 @@ int trajectory_group_levels(int system) {
 
 cudaError_t trajectory_set_tables() {
   cudaError_t e;
-  if ((e = cudaMemcpyToSymbol(c_dop_a, rcmps_dop_a, sizeof(rcmps_dop_a))) != cudaSuccess) return e;
-  if ((e = cudaMemcpyToSymbol(c_dop_b, rcmps_dop_b, sizeof(rcmps_dop_b))) != cudaSuccess) return e;
-  if ((e = cudaMemcpyToSymbol(c_dop_c, rcmps_dop_c, sizeof(rcmps_dop_c))) != cudaSuccess) return e;
-  if ((e = cudaMemcpyToSymbol(c_dop_e5, rcmps_dop_e5, sizeof(rcmps_dop_e5))) != cudaSuccess) return e;
-  if ((e = cudaMemcpyToSymbol(c_dop_e3, rcmps_dop_e3, sizeof(rcmps_dop_e3))) != cudaSuccess) return e;
-  if ((e = cudaMemcpyToSymbol(c_dop_d, rcmps_dop_d, sizeof(rcmps_dop_d))) != cudaSuccess) return e;
+  if ((e = dop853_upload()) != cudaSuccess) return e;
   SysTab tabs[3];
   quartic_table(tabs[0]);
   full_table(tabs[1]);
@@ -1420,8 +1383,7 @@ cudaError_t trajectory_set_tables() {
   quartic_groups(tabs[0]);
   whole_state_groups(tabs[1]);
   whole_state_groups(tabs[2]);
-  if ((e = cudaMemcpyToSymbol(c_sys, tabs, sizeof(tabs))) != cudaSuccess) return e;
-  return cudaMemcpyToSymbol(c_source, rcmps_source_table, sizeof(rcmps_source_table));
+  return cudaMemcpyToSymbol(c_sys, tabs, sizeof(tabs));
 }
 
 template <int SYS>

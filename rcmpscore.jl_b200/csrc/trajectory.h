@@ -23,6 +23,8 @@ struct TrajState {
   const double2 *C, *Ch;              // [Q, R] and its adjoint (all-ODE route)
   const double2* rho;                 // initial value of the rho channels (all-ODE route)
   double2 *y, *prop, *k, *z, *P;      // y, proposed [V]; k [16][V]; z [2][V]; P [V]; V = channels dp^2
+                                      // (quartic system: k [18][V], y and prop its last two, z [3][V],
+                                      // P [16][V], as the tile kernel uses them)
   double2* L;                         // [V] commutator products O X (all-ODE route)
   double2* samples;                   // [npoints][V]
   TrajStats* stats;
@@ -31,6 +33,7 @@ struct TrajState {
   int d;                              // physical bond dimension (d <= dp)
   int z2;                             // quartic system: 1 the packed Z2 error norm (10 (d/2)^2 + 1
                                       // entries), 0 the dense one, -1 refused (no exact Z2 structure)
+  int herm;                           // 1: rho is Hermitian to rounding (hermitian_check)
   // split-precision engine (dp = 64): BF16 slices of the constant operands and their scales,
   // written by split_prep_launch (split_state_bytes() per state)
   const unsigned char* split_g1;      // [rank 4][direction 2][chunk 2] panel^T slices, 48 KB each
@@ -47,6 +50,7 @@ struct TrajControls {
                               // anything else: the default 4)
   int groups = 0;             // CTAs per row block of a state, each for a group of channels: 1, 2 or 4
                               // (0: chosen by the launch, see trajectory_groups)
+  int skip_hermitian = 0;     // leave the states with herm set alone (the tile kernel takes them)
 };
 
 cudaError_t trajectory_set_tables();

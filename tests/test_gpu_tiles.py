@@ -1,0 +1,83 @@
+"""The tile trajectory kernels against the oracle and against the row-block kernel: every tile count
+with ragged and full sizes, one team per channel and one team for all channels (the same bits), the
+packed route with and without whole zero tiles, and a density that is not Hermitian (the row-block
+kernel)."""
+import numpy as np
+import pytest
+
+from oracle import fg_phi4_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+WINDOW, NODES = 1.5, 8
+
+
+def _state(d, z2, seed):
+    from rcmps_b200 import objective
+    from rcmps_b200.batch import random_state, z2_state
+    r, k = (z2_state if z2 else random_state)(d, seed)
+    return r, k, objective.stationary_state(O.left_canonical_q(r, k), r, tolerance=1e-13)[0]
+
+
+def _batch(states, groups=0, symmetry=2):
+    from rcmps_b200 import objective
+    s = objective.settings_from_args(None, half_window=WINDOW, n_quad=NODES, kinetic_nodes=8, symmetry=symmetry,
+                                     trajectory_groups=groups)
+    R, K, rho = zip(*states)
+    E, _, st, C, env = objective.fg_phi4_batch(R, K, rho, [1.0] * len(R), s, return_parts=True)
+    return [(E[i], C[i], env[i], st[i]["accepted"], st[i]["rejected"]) for i in range(len(R))]
+
+
+@pytest.mark.parametrize("d", [1, 2, 15, 16, 17, 32, 33, 48, 49, 64])
+@pytest.mark.parametrize("z2", [False, True])
+def test_quartic_against_the_oracle(gpu_context, d, z2):
+    from rcmps_b200 import objective
+    if z2 and d % 2:
+        pytest.skip("Z2 states have an even D")
+    r, k, rho = _state(d, z2, 60 + d)
+    q = O.left_canonical_q(r, k)
+    o = O.evaluate_quartic(r, q, rho, 1.0, half_window=WINDOW, n_quad=NODES, return_samples=True, packed_z2=z2)
+    g = objective.evaluate_quartic_persistent_trajectory(r, q, rho, 1.0, half_window=WINDOW, n_quad=NODES,
+                                                         return_samples=True, unpacked=not z2)
+    assert (g["stats"]["accepted"], g["stats"]["rejected"]) == (o["stats"]["accepted"], o["stats"]["rejected"])
+    assert abs(g["value"] - o["value"]) <= 1e-11 * max(abs(o["value"]), 1e-3)
+    for out in (g, o):   # the library reports the scalar channel at the endpoint only
+        out["samples"][:-1, -1] = 0
+    for name in ("covector", "environment", "samples"):
+        assert np.linalg.norm(g[name] - o[name]) <= 1e-11 * max(1.0, np.linalg.norm(o[name]))
+
+
+@pytest.mark.parametrize("d,z2", [(80, False), (96, True), (100, False), (128, True)])
+def test_large_tiles_against_the_row_blocks(gpu_context, d, z2):
+    state = _state(d, z2, d)
+    (e0, c0, v0, a0, r0), = _batch([state], groups=1)
+    for n in (1, 4, 9):     # one team per channel, several channels per team, one team
+        for e, c, v, a, r in _batch([state] * n):
+            assert (a, r) == (a0, r0)
+            assert abs(e - e0) <= 1e-12 * abs(e0)
+            assert np.linalg.norm(c - c0) <= 1e-11 * np.linalg.norm(c0)
+            assert np.linalg.norm(v - v0) <= 1e-11 * np.linalg.norm(v0)
+
+
+@pytest.mark.parametrize("d,many", [(9, 24), (16, 24), (24, 40), (32, 40), (40, 5), (48, 20), (50, 4), (64, 12)])
+def test_batch_and_lone_state_give_the_same_bits(gpu_context, d, many):
+    states = [_state(d, i % 2 == 1 and d % 2 == 0, 10 * d + i) for i in range(3)]
+    batch = _batch([states[i % 3] for i in range(many)])
+    for i in range(3):
+        e, c, v, a, r = _batch([states[i]])[0]
+        for j in range(i, many, 3):
+            # the kinetic part's batch sizes may round differently: the environment is the quartic's
+            assert batch[j][3:] == (a, r)
+            assert abs(batch[j][0] - e) <= 1e-13 * abs(e)
+            assert np.linalg.norm(batch[j][1] - c) <= 1e-12 * np.linalg.norm(c)
+
+
+def test_density_that_is_not_hermitian_takes_the_general_equations(gpu_context):
+    r, k, rho = _state(12, False, 3)
+    bent = rho + 1e-9 * (r - r.conj().T)
+    mixed = _batch([(r, k, rho), (r, k, bent)], symmetry=0)
+    alone = [_batch([(r, k, rho)], symmetry=0)[0], _batch([(r, k, bent)], groups=1, symmetry=0)[0]]
+    for got, want in zip(mixed, alone):
+        assert got[3:] == want[3:]
+        assert abs(got[0] - want[0]) <= 1e-13 * abs(want[0])
+        assert np.linalg.norm(got[1] - want[1]) <= 1e-12 * np.linalg.norm(want[1])
