@@ -47,13 +47,14 @@ namespace rcmps {
 //   lsrc/lcoef/lkind: the left insertion c_l ol_a X_a (P_a for ol = R, L_a for the commutator);
 //   rsrc/rcoef: the right insertion c_r X_b ol_b^dag; fixed: 1 fixed0, 2 fixed6;
 //   init: initial value 0, rho (1) or the identity on the physical block (2);
-//   grp_*[k]: the channel groups when a state's rows are also split by channel over 2^k CTAs
-//       (contiguous channel ranges; a G2 pass never straddles two groups), grp_remote[k] when a
-//       left insertion reads P_a of a channel in another group (the CTAs then meet at a cluster
-//       barrier between the G1 products and the G2 epilogues).
+//   grp_*[k]: the channel groups of level k, when a state's rows are also split by channel over
+//       grp_n[k] CTAs (contiguous channel ranges; a G2 pass never straddles two groups), grp_remote[k]
+//       when a left insertion reads P_a or L_a of a channel in another group (the CTAs then meet at a
+//       cluster barrier between the G1 products and the G2 epilogues).
 constexpr int kSysQuartic = 0, kSysFull = 1, kSysPhi1 = 2;
 constexpr int kMaxChannels = 26;
-constexpr int kGroupLevels = 3;   // 1, 2 or 4 channel groups
+constexpr int kGroupLevels = 5;   // 1, 2, 4 channel groups; the all-ODE system also 8 and 14
+constexpr int kMaxGroups = 14;
 struct SysTab {
   int nch, ng1;
   int g1_ch[32], g1_kind[32];
@@ -63,7 +64,8 @@ struct SysTab {
   int fixed[kMaxChannels], init[kMaxChannels];
   double lcoef[kMaxChannels], rcoef[kMaxChannels];
   int grp_levels;                               // group levels available (1: whole-state CTAs only)
-  int grp_first[kGroupLevels][4], grp_count[kGroupLevels][4], grp_remote[kGroupLevels];
+  int grp_n[kGroupLevels], grp_first[kGroupLevels][kMaxGroups], grp_count[kGroupLevels][kMaxGroups],
+      grp_remote[kGroupLevels];
 };
 __constant__ SysTab c_sys[3];
 
@@ -631,7 +633,7 @@ trajectory_kernel(const TrajState* __restrict__ states, const double* __restrict
   // cluster of G x CG CTAs: rows 16 (rank % G) .. + 15 of the channel group rank / G
   const uint32_t nrank = cluster_size();
   const int ngroups = (int)nrank / GE::G;
-  const int glevel = ngroups == 4 ? 2 : ngroups == 2 ? 1 : 0;
+  const int glevel = ngroups == 14 ? 4 : ngroups == 8 ? 3 : ngroups == 4 ? 2 : ngroups == 2 ? 1 : 0;
   const int row0 = (int)(rank % GE::G) * 16;
   const int grp = (int)rank / GE::G;
   const int c0 = c_sys[SYS].grp_first[glevel][grp], c1 = c0 + c_sys[SYS].grp_count[glevel][grp];
@@ -1133,9 +1135,11 @@ static int choose_groups(int nstates, int requested) {
   using GE = Geo<DP, SYS>;
   static int levels = -1;
   if (levels < 0) levels = ENG == 0 ? trajectory_group_levels(SYS) : 1;
+  constexpr int counts[kGroupLevels] = {1, 2, 4, 8, 14};   // groups of each level
   auto allowed = [&](int cg) {
-    const int level = cg == 4 ? 2 : cg == 2 ? 1 : 0;
-    return (cg == 1 || cg == 2 || cg == 4) && level < levels && GE::G * cg <= 16;
+    for (int k = 0; k < levels; ++k)
+      if (counts[k] == cg) return GE::G * cg <= 16;
+    return false;
   };
   // clusters of G x cg CTAs the device holds at once (0 when it cannot place one)
   auto resident = [&](int cg) {
@@ -1156,8 +1160,9 @@ static int choose_groups(int nstates, int requested) {
   }
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return 1;
-  for (int cg = 4; cg > 1; cg /= 2)
-    if (allowed(cg) && (long long)nstates * GE::G * cg <= sms && resident(cg) >= nstates) return cg;
+  for (int k = kGroupLevels - 1; k > 0; --k)
+    if (allowed(counts[k]) && (long long)nstates * GE::G * counts[k] <= sms && resident(counts[k]) >= nstates)
+      return counts[k];
   return 1;
 }
 
@@ -1167,8 +1172,8 @@ static cudaError_t launch_kernel(const TrajState* d_states, int nstates, const d
   using GE = Geo<DP, SYS>;
   cudaError_t e = prepare_kernel<DP, SYS, ENG, NST>();
   if (e != cudaSuccess) return e;
-  const int cg = choose_groups<DP, SYS, ENG>(nstates, ctl.groups);
-  if (cg == 0) return cudaErrorInvalidValue;
+  const int cg = SYS == kSysQuartic ? choose_groups<DP, SYS, ENG>(nstates, ctl.groups) : ctl.groups;
+  if (cg < 1) return cudaErrorInvalidValue;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = launch_config<DP, SYS, ENG>(nstates, GE::G * cg, stream, attr);
   note_launch();
@@ -1319,11 +1324,10 @@ static void phi1_table(SysTab& t) {
   spec_table(t, &spec, 1);
 }
 
-// Channel groups of level k (2^k groups of contiguous channels: first[i], count[i]). The level is
+// Channel groups of level k (ng groups of contiguous channels: first[i], count[i]). The level is
 // kept only when every G2 pass of both tilings lies inside one group; grp_remote[k] records a left
 // insertion whose source channel lies in another group.
-static bool set_groups(SysTab& t, int k, const int* first, const int* count) {
-  const int ng = 1 << k;
+static bool set_groups(SysTab& t, int k, int ng, const int* first, const int* count) {
   int owner[kMaxChannels];
   for (int c = 0; c < t.nch; ++c) owner[c] = -1;
   for (int g = 0, c = 0; g < ng; ++g) {
@@ -1337,7 +1341,8 @@ static bool set_groups(SysTab& t, int k, const int* first, const int* count) {
   int remote = 0;
   for (int c = 0; c < t.nch; ++c)
     if (t.lsrc[c] >= 0 && owner[t.lsrc[c]] != owner[c]) remote = 1;
-  for (int g = 0; g < 4; ++g) {
+  t.grp_n[k] = ng;
+  for (int g = 0; g < kMaxGroups; ++g) {
     t.grp_first[k][g] = g < ng ? first[g] : 0;
     t.grp_count[k][g] = g < ng ? count[g] : 0;
   }
@@ -1347,7 +1352,7 @@ static bool set_groups(SysTab& t, int k, const int* first, const int* count) {
 
 static void whole_state_groups(SysTab& t) {
   const int first[1] = {0}, count[1] = {t.nch};
-  set_groups(t, 0, first, count);
+  set_groups(t, 0, 1, first, count);
   t.grp_levels = 1;
 }
 
@@ -1357,10 +1362,29 @@ static void quartic_groups(SysTab& t) {
   whole_state_groups(t);
   const int f2[2] = {0, 3}, n2[2] = {3, 4};
   const int f4[4] = {0, 2, 3, 5}, n4[4] = {2, 1, 2, 2};
-  if (set_groups(t, 1, f2, n2)) {
+  if (set_groups(t, 1, 2, f2, n2)) {
     t.grp_levels = 2;
-    if (set_groups(t, 2, f4, n4)) t.grp_levels = 3;
+    if (set_groups(t, 2, 4, f4, n4)) t.grp_levels = 3;
   }
+}
+
+// The all-ODE system by direction, then along its G2 pairs. Costs in products: a pair of kinetic1 or
+// phi^4 channels 8, of commutator channels 11 or 12, the last phi^4 channel 4; each level balances the
+// groups' sums (14 groups: one pair each, at most 12 of the 116).
+static void full_groups(SysTab& t) {
+  whole_state_groups(t);
+  const int f2[2] = {0, 13}, n2[2] = {13, 13};
+  const int f4[4] = {0, 6, 13, 19}, n4[4] = {6, 7, 6, 7};
+  const int f8[8] = {0, 4, 6, 10, 13, 17, 19, 23}, n8[8] = {4, 2, 4, 3, 4, 2, 4, 3};
+  const int f14[14] = {0, 2, 4, 6, 8, 10, 12, 13, 15, 17, 19, 21, 23, 25};
+  const int n14[14] = {2, 2, 2, 2, 2, 2, 1, 2, 2, 2, 2, 2, 2, 1};
+  if (!set_groups(t, 1, 2, f2, n2)) return;
+  t.grp_levels = 2;
+  if (!set_groups(t, 2, 4, f4, n4)) return;
+  t.grp_levels = 3;
+  if (!set_groups(t, 3, 8, f8, n8)) return;
+  t.grp_levels = 4;
+  if (set_groups(t, 4, 14, f14, n14)) t.grp_levels = 5;
 }
 
 int trajectory_group_levels(int system) {
@@ -1368,6 +1392,11 @@ int trajectory_group_levels(int system) {
   if (system == kSysQuartic) {
     quartic_table(t);
     quartic_groups(t);
+    return t.grp_levels;
+  }
+  if (system == kSysFull) {
+    full_table(t);
+    full_groups(t);
     return t.grp_levels;
   }
   return 1;
@@ -1381,7 +1410,7 @@ cudaError_t trajectory_set_tables() {
   full_table(tabs[1]);
   phi1_table(tabs[2]);
   quartic_groups(tabs[0]);
-  whole_state_groups(tabs[1]);
+  full_groups(tabs[1]);
   whole_state_groups(tabs[2]);
   return cudaMemcpyToSymbol(c_sys, tabs, sizeof(tabs));
 }
@@ -1446,8 +1475,8 @@ static int groups_sys(int dp, int nstates, int requested) {
 int trajectory_groups(int system, int dp, int nstates, int requested, int engine) {
   if (engine == 1) return 1;
   if (system == kSysQuartic) return groups_sys<kSysQuartic>(dp, nstates, requested);
-  if (system == kSysFull) return groups_sys<kSysFull>(dp, nstates, requested);
-  if (system == kSysPhi1) return groups_sys<kSysPhi1>(dp, nstates, requested);
+  if (system == kSysFull) return groups_sys<kSysFull>(dp, nstates, 0);   // requests are the quartic system's
+  if (system == kSysPhi1) return 1;
   return 0;
 }
 

@@ -48,8 +48,8 @@ struct TrajControls {
   unsigned long long max_ns;  // device-clock watchdog in ns (0: none)
   int ring = 0;               // stages of the FP64 engine's operand ring on the quartic system (2, 3;
                               // anything else: the default 4)
-  int groups = 0;             // CTAs per row block of a state, each for a group of channels: 1, 2 or 4
-                              // (0: chosen by the launch, see trajectory_groups)
+  int groups = 0;             // CTAs per row block of a state, each for a group of channels (quartic
+                              // system: 0 leaves the choice to the launch, see trajectory_groups)
   int skip_hermitian = 0;     // leave the states with herm set alone (the tile kernel takes them)
 };
 
@@ -64,10 +64,10 @@ size_t split_state_bytes();
 void split_state_pointers(unsigned char* block, TrajState& t);   // t.split_* inside `block`
 cudaError_t split_prep_launch(const TrajState* d_states, int nstates, cudaStream_t stream);
 int trajectory_channels(int system);
-// The channel groups a launch of nstates states takes (requested 0: the most, up to 4, that keeps
-// every state's cluster resident at once; 1, 2, 4: the largest supported count up to that one).
-// A state's cluster has dp/16 x groups CTAs (at most 16). Only the FP64 engine on the quartic
-// system groups; everything else takes 1.
+// The channel groups a launch of nstates states takes: the most that keeps every state's cluster
+// resident at once, up to 4 on the quartic system (requested 1, 2, 4: the largest supported count up to
+// that one) and 14 on the all-ODE system. A state's cluster has dp/16 x groups CTAs (at most 16). The
+// split engine and the <phi> system take 1.
 int trajectory_groups(int system, int dp, int nstates, int requested, int engine = 0);
 cudaError_t node_weights_launch(const double* d_points, const double* d_weights, int n, double* d_wj,
                                 cudaStream_t stream);
