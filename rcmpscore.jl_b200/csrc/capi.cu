@@ -723,6 +723,14 @@ int rcmps_fg_phi4_batch_controls(rcmps_context* ctx, int n, const int* dims, con
   kj.stats = kst.data();
   kj.slot = 1;
   kj.memory_share = 0.3;
+  // SMs that the trajectories leave to the kinetic term
+  int busy = 0;
+  for (int dp : {16, 32, 48, 64, 96, 128}) {
+    int count = 0;
+    for (int i = 0; i < n; ++i) count += padded_dim(dims[i]) == dp;
+    if (count) busy = std::max(busy, tile_trajectory_ctas(dp, count));
+  }
+  kj.spare_sms = std::max(16, ctx->sms - busy);
   // The kinetic term runs on its own thread and stream, the quartic term on another. The boundary
   // solve needs only the environment, which the quartic term writes right after its trajectory:
   // the solve starts then and runs while the quartic pullback produces the covector.

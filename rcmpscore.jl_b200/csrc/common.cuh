@@ -228,6 +228,13 @@ RCMPS_DEVICE_INLINE double dsmem_load(const double* p, uint32_t rank) {
   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(remote) : "memory");
   return v;
 }
+// Write a double into the shared memory of CTA `rank` of this cluster (visible there after the next
+// cluster barrier).
+RCMPS_DEVICE_INLINE void dsmem_store_f64(double* p, uint32_t rank, double v) {
+  uint32_t local = smem_u32(p), remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
+}
 RCMPS_DEVICE_INLINE int dsmem_load_int(const int* p, uint32_t rank) {
   uint32_t local = smem_u32(p), remote;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));

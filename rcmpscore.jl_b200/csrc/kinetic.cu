@@ -368,20 +368,27 @@ __global__ void cgs_finish(ArnoldiProblem* __restrict__ probs, int nprob, int j,
 }
 
 // One whole Gram-Schmidt step (both passes of cgs_partial/cgs_subtract and cgs_finish) in one
-// launch: a cluster of G CTAs per problem, each holding its rows of w in shared memory; the
-// projections h_i and the norms are summed across the cluster through distributed shared memory
-// (in chunk order, as the three-launch form sums its partials). The basis is still streamed twice
-// per pass; what goes is four launches and the global round trips between them.
-constexpr int kCgsMaxCluster = 8;
-constexpr int kCgsThreads = 256;
+// launch: a cluster of G CTAs per problem, each holding its rows of w in shared memory. Every CTA
+// writes its projections and norms into the others' shared memory and sums what it got in rank order:
+// two cluster barriers per pass. The basis is streamed twice per pass, from L2 for the few problems
+// that take this form, so bytes in flight set its time: 1024 threads per CTA, up to 16 CTAs per
+// problem, eight loads in flight per thread, the basis rows of the subtraction split over the warps.
+// (8 CTAs of 256 threads: 64.6 us per step at four D = 64 problems and a mean basis of 64.)
+constexpr int kCgsThreads = 1024;
+constexpr int kCgsMaxRows = 4096;   // rows per CTA
+constexpr size_t kCgsMaxShared = 200 * 1024;
 
-__host__ __device__ inline int cgs_cluster(int n) {
-  const int g = (n + CH - 1) / CH;
-  return g < kCgsMaxCluster ? g : kCgsMaxCluster;
+__host__ __device__ inline int cgs_rows(int n, int g) { return ((n + g - 1) / g + 127) / 128 * 128; }
+inline size_t cgs_shared(int n, int g, int j) {
+  return ((size_t)cgs_rows(n, g) + kCgsThreads + (size_t)(g + 1) * (j + 1)) * sizeof(double2);
 }
-__host__ __device__ inline int cgs_rows(int n) {   // rows per CTA, a multiple of 128
-  const int g = cgs_cluster(n);
-  return ((n + g - 1) / g + 127) / 128 * 128;
+// CTAs per problem: 128 rows each, up to 16, and at most max_ctas for all problems where that leaves at
+// least one; fewer when the gathered projections would not fit; 0: this form does not fit.
+inline int cgs_cluster(int n, int j, int nprob, int max_ctas) {
+  int g = n >= 2048 ? 16 : n >= 1024 ? 8 : n >= 512 ? 4 : n >= 256 ? 2 : 1;
+  while (g > 1 && (long long)nprob * g > max_ctas && cgs_rows(n, g / 2) <= kCgsMaxRows) g /= 2;
+  while (g > 1 && cgs_shared(n, g, j) > kCgsMaxShared) g /= 2;
+  return cgs_rows(n, g) <= kCgsMaxRows && cgs_shared(n, g, j) <= kCgsMaxShared ? g : 0;
 }
 
 __global__ void __launch_bounds__(kCgsThreads) cgs_fused(ArnoldiProblem* __restrict__ probs, int nprob, int j) {
@@ -390,26 +397,30 @@ __global__ void __launch_bounds__(kCgsThreads) cgs_fused(ArnoldiProblem* __restr
   // uniform over the cluster (one problem per cluster)
   if (!P.active || P.exhausted || j >= P.target) return;
   extern __shared__ __align__(16) double2 dyn[];
-  const int n = P.n, rows = cgs_rows(n), G = (int)cluster_size(), ch = (int)cluster_rank();
+  const int G = (int)cluster_size(), ch = (int)cluster_rank(), n = P.n, rows = cgs_rows(n, G), m = j + 1;
   double2* w = dyn;                        // [rows]
-  double2* part = dyn + rows;              // [j + 1]: this CTA's projections
-  double2* h = part + (j + 1);             // [j + 1]: the summed projections
+  double2* part = w + rows;                // [kCgsThreads]: the subtraction's partial sums
+  double2* h = part + kCgsThreads;         // [m]: the summed projections
+  double2* gat = h + m;                    // [G][m]: every CTA's projections
   __shared__ double red[kCgsThreads / 32];
-  __shared__ double xch[2];                // this CTA's |w|^2 before / after the current pass
+  __shared__ double nrm_sh[3][16];         // |w|^2 before, after each pass, of every CTA
   const int r0 = ch * rows, r1 = min(n, r0 + rows);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kCgsThreads / 32;
-  auto block_sum = [&](double v) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int nw = kCgsThreads / 32;
+  // the block's sum of v, written into every CTA's nrm_sh[slot]
+  auto share_sum = [&](double v, int slot) {
     v = warp_sum(v);
-    __syncthreads();
     if (lane == 0) red[warp] = v;
     __syncthreads();
-    double t = 0.0;
-    for (int i = 0; i < nw; ++i) t += red[i];
-    return t;
+    if (warp == 0) {
+      double t = 0.0;
+      for (int i = 0; i < nw; ++i) t += red[i];
+      if (lane < G) dsmem_store_f64(&nrm_sh[slot][ch], (uint32_t)lane, t);
+    }
   };
-  auto cluster_total = [&](int slot) {   // sum of xch[slot] over the cluster, in rank order
+  auto total = [&](int slot) {
     double t = 0.0;
-    for (int g = 0; g < G; ++g) t += dsmem_load(&xch[slot], (uint32_t)g);
+    for (int g = 0; g < G; ++g) t += nrm_sh[slot][g];
     return t;
   };
   double s0 = 0.0;
@@ -420,9 +431,12 @@ __global__ void __launch_bounds__(kCgsThreads) cgs_fused(ArnoldiProblem* __restr
     // before the first projection w = L(V_j): kept for the true residuals of the shifted solves
     if (P.LV && r0 + r < r1) P.LV[(size_t)j * P.ldv + r0 + r] = v;
   }
-  s0 = block_sum(s0);
-  if (threadIdx.x == 0) xch[0] = s0;
+  cluster_sync();   // every CTA runs before the others write into it
+  share_sum(s0, 0);
   double before = 0.0, after = 0.0;
+  // subtraction: 128 rows at a time, the basis split over 8 groups of warps
+  const int sr = threadIdx.x & 127, sg = threadIdx.x >> 7;
+  constexpr int ng = kCgsThreads / 128;
   for (int pass = 0; pass < 2; ++pass) {
     // projections of this CTA's rows: a warp takes two basis vectors at a time
     for (int i = warp; i <= j; i += 2 * nw) {
@@ -458,52 +472,55 @@ __global__ void __launch_bounds__(kCgsThreads) cgs_fused(ArnoldiProblem* __restr
       im0 = warp_sum(im0);
       re1 = warp_sum(re1);
       im1 = warp_sum(im1);
-      if (lane == 0) {
-        part[i] = make_double2(re0, im0);
-        if (two) part[i + nw] = make_double2(re1, im1);
+      if (lane < G) {
+        double* to = &gat[(size_t)ch * m + i].x;
+        dsmem_store_f64(to, (uint32_t)lane, re0);
+        dsmem_store_f64(to + 1, (uint32_t)lane, im0);
+        if (two) {
+          to = &gat[(size_t)ch * m + i + nw].x;
+          dsmem_store_f64(to, (uint32_t)lane, re1);
+          dsmem_store_f64(to + 1, (uint32_t)lane, im1);
+        }
       }
     }
     cluster_sync();
-    if (pass == 0) before = cluster_total(0);
+    if (pass == 0) before = total(0);
     for (int i = threadIdx.x; i <= j; i += kCgsThreads) {
       double2 t = make_double2(0, 0);
-      for (int g = 0; g < G; ++g) {
-        t.x += dsmem_load(&part[i].x, (uint32_t)g);
-        t.y += dsmem_load(&part[i].y, (uint32_t)g);
-      }
+      for (int g = 0; g < G; ++g) t = zadd(t, gat[(size_t)g * m + i]);
       h[i] = t;
       if (ch == 0) P.H[(size_t)i * P.kmax + j] = zadd(P.H[(size_t)i * P.kmax + j], t);
     }
-    cluster_sync();   // every CTA has read the others' projections (and xch[0]) before they change
+    __syncthreads();
     double nrm = 0.0;
-    for (int r = threadIdx.x; r < r1 - r0; r += kCgsThreads) {
-      double2 acc = w[r];
-      const double2* v = P.V + r0 + r;
-      int i = 0;
-      for (; i + 3 <= j; i += 4) {
-        double2 x[4];
+    for (int rb = 0; rb < rows; rb += 128) {
+      const int r = rb + sr;
+      double2 acc = make_double2(0, 0);
+      if (r0 + r < r1) {
+        const double2* v = P.V + r0 + r;
+        int i = sg;
+        for (; i + 7 * ng <= j; i += 8 * ng) {
+          double2 x[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) x[u] = v[(size_t)(i + u) * P.ldv];
+          for (int u = 0; u < 8; ++u) x[u] = v[(size_t)(i + u * ng) * P.ldv];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const double2 c = h[i + u];
-          acc.x -= x[u].x * c.x - x[u].y * c.y;
-          acc.y -= x[u].x * c.y + x[u].y * c.x;
+          for (int u = 0; u < 8; ++u) acc = zadd(acc, zmul(x[u], h[i + u * ng]));
         }
+        for (; i <= j; i += ng) acc = zadd(acc, zmul(v[(size_t)i * P.ldv], h[i]));
       }
-      for (; i <= j; ++i) {
-        const double2 x = v[(size_t)i * P.ldv], c = h[i];
-        acc.x -= x.x * c.x - x.y * c.y;
-        acc.y -= x.x * c.y + x.y * c.x;
+      part[threadIdx.x] = acc;
+      __syncthreads();
+      if (sg == 0) {
+        double2 t = w[r];
+        for (int g = 0; g < ng; ++g) t = zsub(t, part[g * 128 + sr]);
+        w[r] = t;
+        nrm += zabs2(t);
       }
-      w[r] = acc;
-      nrm += zabs2(acc);
+      __syncthreads();
     }
-    nrm = block_sum(nrm);
-    if (threadIdx.x == 0) xch[1] = nrm;
+    share_sum(nrm, 1 + pass);
     cluster_sync();
-    after = cluster_total(1);
-    cluster_sync();   // xch[1] is rewritten by the second pass
+    after = total(1 + pass);
     // the second pass only when the first lost more than 1 - 1/sqrt(2) of the norm (uniform)
     if (pass == 0 && after > 0.5 * before) break;
   }
@@ -922,155 +939,179 @@ contract_kernel(ContractArgs a) {
   if (tid == 0 && *flag) atomicExch(a.error_flag + (so >> 1), 1);
 }
 
-__device__ void kmat_mul(double2* C, const double2* A, const double2* B, int dp, double alpha, bool add) {
-  for (int e = threadIdx.x; e < dp * dp; e += blockDim.x) {
-    const int i = e / dp, j = e % dp;
-    double2 s = make_double2(0.0, 0.0);
-    for (int l = 0; l < dp; ++l) s = zadd(s, zmul(A[i * dp + l], B[l * dp + j]));
-    s = zscale(alpha, s);
-    C[e] = add ? zadd(C[e], s) : s;
+// The finalize step of a state and op (kinetic_backend.py:550-583) in four launches spread over the
+// elements; one CTA per state took 6.9 ms at D = 64 (18 products and the 134 MB of solutions through
+// one SM), these take 60 us together. Matrices of (state s, op o) at fin + (s kFinMats + 8 o) dp^2:
+// 0 m, 1 S1, 2 nn, 3 S3, 4 u = sum w X, 5 sa = sum w A, 6 v = sa rho, 7 op^dag sa.
+constexpr int kSumRows = 32, kSumGroups = 8;
+
+// The sums over nodes and node blocks: 32 elements per CTA, the nodes dealt to 8 warps whose sums are
+// added in warp order.
+__global__ void __launch_bounds__(kSumRows* kSumGroups) contract_sum(ContractArgs a, int nblk) {
+  const int so = blockIdx.y, s = so >> 1, op = so & 1;
+  const int dp = a.dp, MAT = dp * dp;
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int e = blockIdx.x * kSumRows + lane;
+  const double2 *X = a.X[so] + e, *A = a.A[so] + e;
+  const double2* opm = op ? a.comm + (size_t)s * 2 * MAT : a.R[s];
+  double2 sum[6] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}};
+  double vpart = 0.0;
+  for (int b = g; b < nblk; b += kSumGroups) {
+    const double2* pp = a.partial + (((size_t)so * nblk + b) * 4) * MAT + e;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sum[q] = zadd(sum[q], pp[(size_t)q * MAT]);
   }
+  // Re tr(op X) = sum_ij Re(op_ji X_ij)
+  const double2 opji = opm[(e % dp) * dp + e / dp];
+#pragma unroll 4
+  for (int c = g; c < a.nodes; c += kSumGroups) {
+    const double w = a.weights[c];
+    const double2 xv = X[(size_t)c * MAT], av = A[(size_t)c * MAT];
+    sum[4] = zaxpy(w, xv, sum[4]);
+    sum[5] = zaxpy(w, av, sum[5]);
+    vpart += w * (opji.x * xv.x - opji.y * xv.y);
+  }
+  __shared__ double2 sh[kSumGroups][6][kSumRows];
+  __shared__ double vsh[kSumGroups];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) sh[g][q][lane] = sum[q];
+  vpart = warp_sum(vpart);
+  if (lane == 0) vsh[g] = vpart;
   __syncthreads();
+  const int slot[6] = {0, 1, 2, 3, 4, 5};
+  if (g < 6) {
+    double2 t = sh[0][g][lane];
+    for (int i = 1; i < kSumGroups; ++i) t = zadd(t, sh[i][g][lane]);
+    a.fin[((size_t)s * kFinMats + 8 * op + slot[g]) * MAT + e] = t;
+  }
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int i = 0; i < kSumGroups; ++i) t += vsh[i];
+    a.vpart[(size_t)so * gridDim.x + blockIdx.x] = t;
+  }
 }
 
-// One CTA per state: value, covector and environment of both kinetic terms
-// (kinetic_backend.py:550-583).
-__global__ void contract_finalize(ContractArgs a, int nblk) {
-  const int s = blockIdx.x;
-  const int dp = a.dp, MAT = dp * dp;
-  const double2 *Q = a.Q[s], *Qh = a.Qh[s], *R = a.R[s], *Rh = a.Rh[s], *rho = a.rho[s];
-  double2* t = a.fin + (size_t)s * 12 * MAT;
-  double2 *m = t, *S1 = t + MAT, *nn = t + 2 * MAT, *S3 = t + 3 * MAT, *u = t + 4 * MAT, *sa = t + 5 * MAT,
-          *v = t + 6 * MAT, *T1 = t + 7 * MAT, *T2 = t + 8 * MAT, *cov = t + 9 * MAT, *env = t + 10 * MAT,
-          *opm = t + 11 * MAT;
-  __shared__ double red[32];
-  double value = 0.0;
-  for (int e = threadIdx.x; e < MAT; e += blockDim.x) {
-    cov[e] = make_double2(0, 0);
-    env[e] = make_double2(0, 0);
+// v = sa rho
+__global__ void contract_v(ContractArgs a) {
+  const int so = blockIdx.y, s = so >> 1, dp = a.dp, MAT = dp * dp;
+  double2* f = a.fin + ((size_t)s * kFinMats + 8 * (so & 1)) * MAT;
+  const double2 *sa = f + 5 * (size_t)MAT, *rho = a.rho[s];
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, i = e / dp, j = e % dp;
+  double2 t = make_double2(0, 0);
+#pragma unroll 8
+  for (int l = 0; l < dp; ++l) t = zadd(t, zmul(sa[i * dp + l], rho[l * dp + j]));
+  f[6 * (size_t)MAT + e] = t;
+}
+
+// Whole rows per CTA (blockDim = dp x rows):
+//   op R:     m = S0 - S1 R^dag + u,  nn = S2 - R S3 + v
+//   op [Q,R]: m = S0 - (S1 + R u - u R) R^dag + u Q - Q u,
+//             nn = S2 - R S3 + Q^dag v - v Q^dag - (R v) R^dag + (R R^dag) v
+//   env = op^dag sa
+__global__ void contract_rows(ContractArgs a) {
+  const int so = blockIdx.y, s = so >> 1, op = so & 1, dp = a.dp, MAT = dp * dp;
+  const double2 *Q = a.Q[s], *Qh = a.Qh[s], *R = a.R[s], *Rh = a.Rh[s];
+  double2* f = a.fin + ((size_t)s * kFinMats + 8 * op) * MAT;
+  double2 *m = f, *nn = f + 2 * (size_t)MAT, *env = f + 7 * (size_t)MAT;
+  const double2 *S1 = f + MAT, *S3 = f + 3 * (size_t)MAT, *u = f + 4 * (size_t)MAT, *sa = f + 5 * (size_t)MAT,
+                *v = f + 6 * (size_t)MAT;
+  const double2* oph = op ? a.comm + ((size_t)s * 2 + 1) * MAT : Rh;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, i = e / dp, j = e % dp, row = (threadIdx.x / dp) * dp;
+  const double2 z = make_double2(0, 0);
+  __shared__ double2 w[128], y1[128], y2[128];
+  double2 rs3 = z, ev = z, t1 = z, t2 = z, uq = z, qu = z, qv = z, vq = z, rv = z, rr = z;
+#pragma unroll 2
+  for (int l = 0; l < dp; ++l) {
+    const int il = i * dp + l, lj = l * dp + j;
+    rs3 = zadd(rs3, zmul(R[il], S3[lj]));
+    ev = zadd(ev, zmul(oph[il], sa[lj]));
+    if (op) {
+      t1 = zadd(t1, zmul(R[il], u[lj]));
+      t2 = zadd(t2, zmul(u[il], R[lj]));
+      uq = zadd(uq, zmul(u[il], Q[lj]));
+      qu = zadd(qu, zmul(Q[il], u[lj]));
+      qv = zadd(qv, zmul(Qh[il], v[lj]));
+      vq = zadd(vq, zmul(v[il], Qh[lj]));
+      rv = zadd(rv, zmul(R[il], v[lj]));
+      rr = zadd(rr, zmul(R[il], Rh[lj]));
+    }
   }
+  w[threadIdx.x] = zadd(S1[e], zsub(t1, t2));
+  y1[threadIdx.x] = rv;
+  y2[threadIdx.x] = rr;
   __syncthreads();
-  for (int op = 0; op < 2; ++op) {
-    const int so = 2 * s + op;
-    const double2 *X = a.X[so], *Aa = a.A[so];
-    // op matrix: R or C = QR - RQ
-    if (op == 0) {
-      for (int e = threadIdx.x; e < MAT; e += blockDim.x) opm[e] = R[e];
-      __syncthreads();
-    } else {
-      kmat_mul(opm, Q, R, dp, 1.0, false);
-      kmat_mul(opm, R, Q, dp, -1.0, true);
+  double2 wr = z, yr = z, zv = z;
+#pragma unroll 4
+  for (int l = 0; l < dp; ++l) {
+    const int lj = l * dp + j;
+    wr = zadd(wr, zmul(w[row + l], Rh[lj]));
+    if (op) {
+      yr = zadd(yr, zmul(y1[row + l], Rh[lj]));
+      zv = zadd(zv, zmul(y2[row + l], v[lj]));
     }
-    double vpart = 0.0;
-    for (int e = threadIdx.x; e < MAT; e += blockDim.x) {
-      double2 sm[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-      for (int b = 0; b < nblk; ++b) {
-        const double2* pp = a.partial + (((size_t)so * nblk + b) * 4) * MAT;
-        for (int q = 0; q < 4; ++q) sm[q] = zadd(sm[q], pp[q * MAT + e]);
-      }
-      m[e] = sm[0];
-      S1[e] = sm[1];
-      nn[e] = sm[2];
-      S3[e] = sm[3];
-      double2 uu = make_double2(0, 0), ss = make_double2(0, 0);
-      const int i = e / dp, j = e % dp;
-      const double2 opji = opm[j * dp + i];
-      for (int c = 0; c < a.nodes; ++c) {
-        const double w = a.weights[c];
-        const double2 xv = X[(size_t)c * MAT + e];
-        uu = zaxpy(w, xv, uu);
-        ss = zaxpy(w, Aa[(size_t)c * MAT + e], ss);
-        // Re tr(op X) = sum_ij Re(op_ji X_ij)
-        vpart += w * (opji.x * xv.x - opji.y * xv.y);
-      }
-      u[e] = uu;
-      sa[e] = ss;
-    }
-    __syncthreads();
-    vpart = warp_sum(vpart);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = vpart;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double tot = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += red[w];
-      value += tot;
-    }
-    __syncthreads();
-    // m = S0 - S1 R^dag (+ u terms), nn = S2 - R S3 (+ v terms), v = sa rho
-    kmat_mul(m, S1, Rh, dp, -1.0, true);
-    kmat_mul(nn, R, S3, dp, -1.0, true);
-    kmat_mul(v, sa, rho, dp, 1.0, false);
-    if (op == 0) {
-      for (int e = threadIdx.x; e < MAT; e += blockDim.x) {
-        m[e] = zadd(m[e], u[e]);
-        nn[e] = zadd(nn[e], v[e]);
-      }
-      __syncthreads();
-    } else {
-      // m += u Q - Q u - R u R^dag + u R R^dag;  nn += Q^dag v - v Q^dag - R v R^dag + R R^dag v
-      kmat_mul(m, u, Q, dp, 1.0, true);
-      kmat_mul(m, Q, u, dp, -1.0, true);
-      kmat_mul(T1, R, u, dp, 1.0, false);
-      kmat_mul(m, T1, Rh, dp, -1.0, true);
-      kmat_mul(T1, u, R, dp, 1.0, false);
-      kmat_mul(m, T1, Rh, dp, 1.0, true);
-      kmat_mul(nn, Qh, v, dp, 1.0, true);
-      kmat_mul(nn, v, Qh, dp, -1.0, true);
-      kmat_mul(T2, R, v, dp, 1.0, false);
-      kmat_mul(nn, T2, Rh, dp, -1.0, true);
-      kmat_mul(T2, R, Rh, dp, 1.0, false);
-      kmat_mul(nn, T2, v, dp, 1.0, true);
-    }
-    // env_op = op^dag sa
-    for (int e = threadIdx.x; e < MAT; e += blockDim.x) {
-      const int i = e / dp, j = e % dp;
-      double2 acc = make_double2(0, 0);
-      for (int l = 0; l < dp; ++l) acc = zadd(acc, zmul(zconj(opm[l * dp + i]), sa[l * dp + j]));
-      T1[e] = acc;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < MAT; e += blockDim.x) {
-      const int i = e / dp, j = e % dp;
-      cov[e] = zadd(cov[e], zscale(0.5, zadd(m[e], zconj(nn[j * dp + i]))));
-      env[e] = zadd(env[e], zscale(0.5, zadd(T1[e], zconj(T1[j * dp + i]))));
-    }
-    __syncthreads();
   }
-  if (threadIdx.x == 0) a.value_out[s] = value;
+  if (op) {
+    m[e] = zadd(zsub(m[e], wr), zsub(uq, qu));
+    nn[e] = zadd(zadd(zsub(nn[e], rs3), zsub(qv, vq)), zsub(zv, yr));
+  } else {
+    m[e] = zadd(zsub(m[e], wr), u[e]);
+    nn[e] = zadd(zsub(nn[e], rs3), v[e]);
+  }
+  env[e] = ev;
+}
+
+// covector = sum_op (m + nn^dag)/2, environment = sum_op Herm(env), value
+__global__ void contract_combine(ContractArgs a, int nvpart) {
+  const int s = blockIdx.y, dp = a.dp, MAT = dp * dp;
+  double2* f = a.fin + (size_t)s * kFinMats * MAT;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, et = (e % dp) * dp + e / dp;
+  double2 cov = make_double2(0, 0), env = cov;
+  for (int op = 0; op < 2; ++op) {
+    const double2* t = f + (size_t)8 * op * MAT;
+    cov = zadd(cov, zscale(0.5, zadd(t[e], zconj(t[2 * (size_t)MAT + et]))));
+    env = zadd(env, zscale(0.5, zadd(t[7 * (size_t)MAT + e], zconj(t[7 * (size_t)MAT + et]))));
+  }
+  f[(size_t)kFinCov * MAT + e] = cov;
+  f[(size_t)kFinEnv * MAT + e] = env;
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
+    double t = 0.0;
+    for (int i = threadIdx.x; i < 2 * nvpart; i += 32) t += a.vpart[(size_t)2 * s * nvpart + i];
+    t = warp_sum(t);
+    if (threadIdx.x == 0) a.value_out[s] = t;
+  }
 }
 
 // ======================================================================= problem set-up
 // Per state: the commutator C = QR - RQ and the four right-hand sides
 //   R fwd: rho R^dag, R adj: R^dag, C fwd: rho C^dag, C adj: C^dag (kinetic_backend.py:281-284).
-__global__ void kinetic_rhs_kernel(KineticSetup a) {
-  const int s = blockIdx.x, dp = a.dp, MAT = dp * dp;
-  const double2 *Q = a.ops + (size_t)s * a.ops_stride, *R = Q + 2 * MAT, *rho = Q + 7 * MAT;
+// One element per thread: first C, C^dag and the right-hand sides without a product, then rho op^dag.
+__global__ void kinetic_comm_kernel(KineticSetup a) {
+  const int s = blockIdx.y, dp = a.dp, MAT = dp * dp;
+  const double2 *Q = a.ops + (size_t)s * a.ops_stride, *R = Q + 2 * MAT;
   double2* c = a.comm + (size_t)s * 2 * MAT;   // C, C^dag
   double2* rhs = a.rhs + (size_t)s * 4 * MAT;
-  for (int e = threadIdx.x; e < MAT; e += blockDim.x) {
-    const int i = e / dp, j = e % dp;
-    double2 v = make_double2(0, 0);
-    for (int l = 0; l < dp; ++l) v = zadd(v, zsub(zmul(Q[i * dp + l], R[l * dp + j]), zmul(R[i * dp + l], Q[l * dp + j])));
-    c[e] = v;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, i = e / dp, j = e % dp, et = j * dp + i;
+  double2 v = make_double2(0, 0);
+#pragma unroll 4
+  for (int l = 0; l < dp; ++l) v = zadd(v, zsub(zmul(Q[i * dp + l], R[l * dp + j]), zmul(R[i * dp + l], Q[l * dp + j])));
+  c[e] = v;
+  c[MAT + et] = zconj(v);
+  rhs[MAT + et] = zconj(R[e]);
+  rhs[3 * MAT + et] = zconj(v);
+}
+__global__ void kinetic_rhs_kernel(KineticSetup a) {
+  const int s = blockIdx.y, dp = a.dp, MAT = dp * dp;
+  const double2* rho = a.ops + (size_t)s * a.ops_stride + 7 * MAT;
+  double2* rhs = a.rhs + (size_t)s * 4 * MAT;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, i = e / dp, j = e % dp;
+  double2 a0 = make_double2(0, 0), a2 = make_double2(0, 0);
+#pragma unroll 4
+  for (int l = 0; l < dp; ++l) {
+    a0 = zadd(a0, zmul(rho[i * dp + l], rhs[MAT + l * dp + j]));
+    a2 = zadd(a2, zmul(rho[i * dp + l], rhs[3 * MAT + l * dp + j]));
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < MAT; e += blockDim.x) {
-    const int i = e / dp, j = e % dp;
-    c[MAT + e] = zconj(c[j * dp + i]);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < MAT; e += blockDim.x) {
-    const int i = e / dp, j = e % dp;
-    double2 a0 = make_double2(0, 0), a2 = make_double2(0, 0);
-    for (int l = 0; l < dp; ++l) {
-      a0 = zadd(a0, zmul(rho[i * dp + l], zconj(R[j * dp + l])));
-      a2 = zadd(a2, zmul(rho[i * dp + l], c[MAT + l * dp + j]));
-    }
-    rhs[e] = a0;
-    rhs[MAT + e] = zconj(R[j * dp + i]);
-    rhs[2 * MAT + e] = a2;
-    rhs[3 * MAT + e] = c[MAT + e];
-  }
+  rhs[e] = a0;
+  rhs[2 * MAT + e] = a2;
 }
 
 // residual-check tasks -> per-problem worst relative residual
@@ -1160,11 +1201,13 @@ cudaError_t cgs_step_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, cu
   return cudaGetLastError();
 }
 
-cudaError_t cgs_fused_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, cudaStream_t s) {
+cudaError_t cgs_fused_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int max_ctas, cudaStream_t s) {
   if (nprob == 0) return cudaSuccess;
-  const int g = cgs_cluster(n), rows = cgs_rows(n);
-  const size_t smem = ((size_t)rows + 2 * (size_t)(j + 1)) * sizeof(double2);
-  cudaError_t e = cudaFuncSetAttribute(cgs_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int g = cgs_cluster(n, j, nprob, max_ctas);
+  if (g == 0) return cudaErrorInvalidValue;
+  const size_t smem = cgs_shared(n, g, j);
+  cudaError_t e = cudaFuncSetAttribute(cgs_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgsMaxShared);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(cgs_fused, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g, nprob, 1);
@@ -1182,11 +1225,17 @@ cudaError_t cgs_fused_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, c
   return cudaLaunchKernelEx(&cfg, cgs_fused, d_probs, nprob, j);
 }
 
-cudaError_t gram_schmidt_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int sms, cudaStream_t s) {
-  // few problems: the step is latency-bound and one clustered launch wins; a large batch streams
-  // the basis from HBM on whatever SMs the concurrent trajectory leaves, where the independent
-  // CTAs of the three-kernel form keep those SMs busier than clusters waiting at their barriers
-  if ((long long)nprob * cgs_cluster(n) <= 2ll * sms) return cgs_fused_launch(d_probs, nprob, j, n, s);
+cudaError_t gram_schmidt_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int sms, int spare, cudaStream_t s) {
+  // Few problems: the step is latency-bound and one clustered launch wins. Its CTAs take an SM each and
+  // a cluster one GPC, so beside a trajectory that leaves `spare` SMs it takes half of those: clusters
+  // of 16 beside a lone D = 64 trajectory (112 SMs) found one GPC and ran one after another (kinetic
+  // term 47 ms; 10 ms alone). A large batch streams the basis from HBM on whatever SMs the concurrent
+  // trajectory leaves, where the independent CTAs of the three-kernel form keep those SMs busier than
+  // clusters waiting at their barriers.
+  const int few = (n + CH - 1) / CH < 8 ? (n + CH - 1) / CH : 8;
+  const int limit = spare >= sms ? sms : spare / 2;
+  if ((long long)nprob * few <= 2ll * sms && cgs_cluster(n, j, nprob, limit))
+    return cgs_fused_launch(d_probs, nprob, j, n, limit, s);
   return cgs_step_launch(d_probs, nprob, j, n, s);
 }
 
@@ -1236,8 +1285,11 @@ cudaError_t residual_reduce_launch(ArnoldiProblem* d_probs, int nprob, const dou
 }
 
 cudaError_t kinetic_rhs_launch(const KineticSetup& a, int nstates, cudaStream_t s) {
+  const dim3 grid(a.dp * a.dp / 128, nstates);
   note_launch();
-  kinetic_rhs_kernel<<<nstates, 256, 0, s>>>(a);
+  kinetic_comm_kernel<<<grid, 128, 0, s>>>(a);
+  note_launch();
+  kinetic_rhs_kernel<<<grid, 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -1265,8 +1317,15 @@ cudaError_t contract_launch(const ContractArgs& a, int nblk, cudaStream_t s) {
     default: return cudaErrorInvalidValue;
   }
   if (e != cudaSuccess) return e;
+  const int mat = a.dp * a.dp, rows = a.dp >= 128 ? 1 : 128 / a.dp, nvpart = mat / kSumRows;
   note_launch();
-  contract_finalize<<<a.nstates, 256, 0, s>>>(a, nblk);
+  contract_sum<<<dim3(nvpart, 2 * a.nstates), kSumRows * kSumGroups, 0, s>>>(a, nblk);
+  note_launch();
+  contract_v<<<dim3(mat / 128, 2 * a.nstates), 128, 0, s>>>(a);
+  note_launch();
+  contract_rows<<<dim3(a.dp / rows, 2 * a.nstates), a.dp * rows, 0, s>>>(a);
+  note_launch();
+  contract_combine<<<dim3(mat / 128, a.nstates), 128, 0, s>>>(a, nvpart);
   return cudaGetLastError();
 }
 

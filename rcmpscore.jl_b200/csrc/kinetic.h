@@ -58,6 +58,8 @@ struct KineticSetup {
   double2* rhs;              // [state][4 dp^2]
 };
 
+constexpr int kFinMats = 18, kFinCov = 16, kFinEnv = 17;   // finalize matrices of a state (contract_launch)
+
 struct ContractArgs {
   int dp, nstates, nodes, nodes_per_block;
   const double2* const* X;   // [2 nstates]: forward solutions of (state, op)
@@ -70,7 +72,9 @@ struct ContractArgs {
   const double* weights;     // [nodes]
   const double* shifts;      // [nodes]
   double2* partial;          // [2 nstates][nblk][4][dp^2]
-  double2* fin;              // [nstates][12 dp^2]; covector at 9, environment at 10
+  const double2* comm;       // [nstates][2 dp^2]: C, C^dag
+  double2* fin;              // [nstates][kFinMats dp^2]; covector at kFinCov, environment at kFinEnv
+  double* vpart;             // [2 nstates][dp^2 / 32] partial sums of the value
   double* value_out;         // [nstates]
   int* error_flag;           // [nstates]
 };
@@ -80,10 +84,12 @@ cudaError_t arnoldi_tasks_launch(const ArnoldiProblem* d_probs, int nprob, int j
                                 cudaStream_t s);
 cudaError_t arnoldi_start_launch(ArnoldiProblem* d_probs, int nprob, cudaStream_t s);
 cudaError_t cgs_step_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, cudaStream_t s);
-// The same Gram-Schmidt step in one launch (a cluster per problem; no partial or norm arrays).
-cudaError_t cgs_fused_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, cudaStream_t s);
-// The Gram-Schmidt step by whichever of the two forms suits the batch (sms: the device's SMs).
-cudaError_t gram_schmidt_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int sms, cudaStream_t s);
+// The same Gram-Schmidt step in one launch (a cluster per problem, max_ctas for all of them where that
+// leaves at least one; no partial or norm arrays).
+cudaError_t cgs_fused_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int max_ctas, cudaStream_t s);
+// The Gram-Schmidt step by whichever of the two forms suits the batch (sms: the device's SMs; spare:
+// those that work running beside this leaves free).
+cudaError_t gram_schmidt_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int sms, int spare, cudaStream_t s);
 // W = L(V_j) (or L(Z_j)) of step j of every problem still extending, the task built in the kernel.
 cudaError_t lindblad_arnoldi_launch(int dp, const ArnoldiProblem* d_probs, int nprob, int j, cudaStream_t s);
 cudaError_t hessenberg_launch(ArnoldiProblem* d_probs, int nprob, const double* d_shifts, int nshift,

@@ -38,7 +38,7 @@ size_t kinetic_state_bytes(int dp, int kmax, int nshift) {
   b += 4 * ((size_t)(2 * kmax + 1) * mat + (size_t)(kmax + 1) * kmax * 16 + mat + (size_t)nchunk * (kmax + 1) * 16 +
             (size_t)nshift * kmax * 16 + (size_t)nshift * mat);      // per problem (V, L(V), H, ...)
   b += 4 * (size_t)nshift * ((dp * dp + 63) / 64) * 8;
-  b += 2 * (size_t)nblk * 4 * mat + 12 * mat;                        // contraction
+  b += 2 * (size_t)nblk * 4 * mat + kFinMats * mat + mat / 32;       // contraction
   return b + 4096;
 }
 }  // namespace
@@ -109,7 +109,8 @@ int kinetic_run(rcmps_context* ctx, KineticJob& job, cudaStream_t stream) {
       const size_t o_mtasks = L.add(NP * sizeof(LindbladTask));
       const size_t o_res = L.add((size_t)NP * nshift * ntile * 8);
       const size_t o_cpart = L.add((size_t)2 * n * nblk * 4 * mat * 16);
-      const size_t o_fin = L.add((size_t)n * 12 * mat * 16);
+      const size_t o_fin = L.add((size_t)n * kFinMats * mat * 16);
+      const size_t o_vpart = L.add((size_t)2 * n * (mat / 32) * 8);
       const size_t o_val = L.add(n * 8);
       const size_t o_ptrs = L.add((size_t)(4 * n + 5 * n) * sizeof(void*));
       const size_t o_scr = L.add(scratch_budget);
@@ -232,7 +233,7 @@ int kinetic_run(rcmps_context* ctx, KineticJob& job, cudaStream_t stream) {
         e = cudaMemcpyAsync(d_probs, hp, NP * sizeof(ArnoldiProblem), cudaMemcpyHostToDevice, stream);
         for (int j = jlo; j < jhi && !e; ++j) {
           e = lindblad_arnoldi_launch(dp, d_probs, NP, j, stream);
-          if (!e) e = gram_schmidt_launch(d_probs, NP, j, nvec, ctx->sms, stream);
+          if (!e) e = gram_schmidt_launch(d_probs, NP, j, nvec, ctx->sms, job.spare_sms > 0 ? job.spare_sms : ctx->sms, stream);
         }
         // ---- projected solves of every open problem
         int kcur = 1;
@@ -359,16 +360,18 @@ int kinetic_run(rcmps_context* ctx, KineticJob& job, cudaStream_t stream) {
       ca.weights = (double*)P(o_weight);
       ca.shifts = (double*)P(o_shift);
       ca.partial = (double2*)P(o_cpart);
+      ca.comm = d_comm;
       ca.fin = (double2*)P(o_fin);
+      ca.vpart = (double*)P(o_vpart);
       ca.value_out = (double*)P(o_val);
       ca.error_flag = d_flags + NP;
       if (!e) e = contract_launch(ca, nblk, stream);
-      // outputs: covector (fin slot 9) and environment (slot 10) of each state, unpadded
+      // outputs: covector and environment of each state, unpadded
       if (!e && job.covector)
-        e = launch_unpad_acc(reinterpret_cast<double*>((double2*)P(o_fin) + 9 * mat), (long long)(12 * mat), dp,
+        e = launch_unpad_acc(reinterpret_cast<double*>((double2*)P(o_fin) + kFinCov * mat), (long long)(kFinMats * mat), dp,
                              (long long*)P(o_off), (int*)P(o_dims), job.covector, n, job.accumulate, stream);
       if (!e && job.environment)
-        e = launch_unpad_acc(reinterpret_cast<double*>((double2*)P(o_fin) + 10 * mat), (long long)(12 * mat), dp,
+        e = launch_unpad_acc(reinterpret_cast<double*>((double2*)P(o_fin) + kFinEnv * mat), (long long)(kFinMats * mat), dp,
                              (long long*)P(o_off), (int*)P(o_dims), job.environment, n, job.accumulate, stream);
       if (!e && job.value)
         e = launch_scatter_values((double*)P(o_val), n, (int*)P(o_idx), job.value, job.accumulate, stream);

@@ -17,6 +17,7 @@ struct KineticJob {
   double* environment = nullptr;        // device packed, optional
   rcmps_state_stats* stats = nullptr;   // host [n]
   bool accumulate = false;
+  int spare_sms = 0;                    // SMs that the work beside this job leaves free (0: all)
   int slot = 1;
   double memory_share = 0.7;
 };

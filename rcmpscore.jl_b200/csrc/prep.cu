@@ -32,12 +32,12 @@ __global__ void unpad_kernel(const double2* __restrict__ src, long long stride, 
   }
 }
 
-// Q = -iK - R^dag R / 2, and the derived operators of one padded state (one CTA per state).
+// Q = -iK - R^dag R / 2, and the derived operators of the padded states, one element per thread.
 // Layout of `ops` per state: Q, Qh, R, Rh, fixed0, fixed6, S, rho (8 matrices of dp^2).
 __global__ void prepare_kernel(const double2* __restrict__ R, const double2* __restrict__ K,
                                const double2* __restrict__ rho, double2* __restrict__ ops, int dp,
                                long long in_stride, long long ops_stride) {
-  const int s = blockIdx.x;
+  const int s = blockIdx.y;
   const int n = dp * dp;
   const double2* r = R + s * in_stride;
   const double2* k = K + s * in_stride;
@@ -45,30 +45,27 @@ __global__ void prepare_kernel(const double2* __restrict__ R, const double2* __r
   double2* o = ops + s * ops_stride;
   double2 *Q = o, *Qh = o + n, *Ro = o + 2 * n, *Rh = o + 3 * n, *F0 = o + 4 * n, *F6 = o + 5 * n,
           *S = o + 6 * n, *P = o + 7 * n;
-  for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    const int i = e / dp, j = e % dp;
-    double2 rr = make_double2(0.0, 0.0);   // (R^dag R)_ij = sum_l conj(R_li) R_lj
-    double2 rp = make_double2(0.0, 0.0);   // (R rho)_ij
-    double2 pr = make_double2(0.0, 0.0);   // (rho R^dag)_ij = sum_l rho_il conj(R_jl)
-    for (int l = 0; l < dp; ++l) {
-      rr = zadd(rr, zmul(zconj(r[l * dp + i]), r[l * dp + j]));
-      rp = zadd(rp, zmul(r[i * dp + l], p[l * dp + j]));
-      pr = zadd(pr, zmul(p[i * dp + l], zconj(r[j * dp + l])));
-    }
-    const double2 kij = k[e];
-    Q[e] = make_double2(kij.y - 0.5 * rr.x, -kij.x - 0.5 * rr.y);   // -i K - R^dag R / 2
-    Ro[e] = r[e];
-    Rh[e] = zconj(r[j * dp + i]);
-    F0[e] = zadd(rp, pr);
-    F6[e] = zscale(4.0, zadd(r[e], zconj(r[j * dp + i])));
-    S[e] = zadd(zconj(r[e]), r[j * dp + i]);
-    P[e] = p[e];
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = e / dp, j = e % dp, et = j * dp + i;
+  double2 rr = make_double2(0.0, 0.0);   // (R^dag R)_ij = sum_l conj(R_li) R_lj
+  double2 rp = make_double2(0.0, 0.0);   // (R rho)_ij
+  double2 pr = make_double2(0.0, 0.0);   // (rho R^dag)_ij = sum_l rho_il conj(R_jl)
+#pragma unroll 4
+  for (int l = 0; l < dp; ++l) {
+    rr = zadd(rr, zmul(zconj(r[l * dp + i]), r[l * dp + j]));
+    rp = zadd(rp, zmul(r[i * dp + l], p[l * dp + j]));
+    pr = zadd(pr, zmul(p[i * dp + l], zconj(r[j * dp + l])));
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    const int i = e / dp, j = e % dp;
-    Qh[e] = zconj(Q[j * dp + i]);
-  }
+  const double2 kij = k[e];
+  const double2 q = make_double2(kij.y - 0.5 * rr.x, -kij.x - 0.5 * rr.y);   // -i K - R^dag R / 2
+  Q[e] = q;
+  Qh[et] = zconj(q);
+  Ro[e] = r[e];
+  Rh[e] = zconj(r[et]);
+  F0[e] = zadd(rp, pr);
+  F6[e] = zscale(4.0, zadd(r[e], zconj(r[et])));
+  S[e] = zadd(zconj(r[e]), r[et]);
+  P[e] = p[e];
 }
 
 // Operators of the commutator channels of the all-ODE route: C = Q R - R Q at slot kC and
@@ -306,7 +303,7 @@ cudaError_t launch_prepare(const double* R, const double* K, const double* rho, 
                            long long in_stride, long long ops_stride, int nstates, cudaStream_t stream) {
   if (nstates == 0) return cudaSuccess;
   note_launch();
-  prepare_kernel<<<nstates, 256, 0, stream>>>(reinterpret_cast<const double2*>(R),
+  prepare_kernel<<<dim3(dp * dp / 64, nstates), 64, 0, stream>>>(reinterpret_cast<const double2*>(R),
                                               reinterpret_cast<const double2*>(K),
                                               reinterpret_cast<const double2*>(rho),
                                               reinterpret_cast<double2*>(ops), dp, in_stride, ops_stride);

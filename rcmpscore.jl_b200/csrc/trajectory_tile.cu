@@ -142,12 +142,6 @@ struct Smem {
   }
 };
 
-__device__ __forceinline__ void dsmem_store(double* p, uint32_t rank, double v) {
-  uint32_t local = smem_u32(p), remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
-}
-
 __device__ __forceinline__ void flag_release(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -233,7 +227,7 @@ __device__ __forceinline__ void share_dec(Dec* shared, const Dec& d) {
   constexpr int words = sizeof(Dec) / 8;
   for (int i = lane; i < words * (NR - 1); i += 32) {
     double* w = reinterpret_cast<double*>(shared) + i % words;
-    dsmem_store(w, 1 + i / words, *w);
+    dsmem_store_f64(w, 1 + i / words, *w);
   }
 }
 
@@ -924,7 +918,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
                                     [&](int q, int c, int i) { return s_we[(q * SM::NC + (LONE ? 0 : c)) * G::NW + i]; });
       if constexpr (SM::GLOBAL_REC) sy->crec[team][rank][tid] = x;
       else if constexpr (NR == 1) s_gat[tid] = x;
-      else dsmem_store(s_gat + rank * SM::NREC + tid, 0, x);
+      else dsmem_store_f64(s_gat + rank * SM::NREC + tid, 0, x);
     }
     team_sync();
     if (rank == 0 && warp == 0) {
@@ -1345,7 +1339,7 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
       const double x = record_entry(S, tid, W::PARTS, 0, kChannels, h, ctl_in.max_ns && global_ns() - t_start >= ctl_in.max_ns,
                                     [&](int q, int ch, int i) { return s_we[(q * kChannels + ch) * W::PARTS + i]; });
       if constexpr (NR == 1) s_gat[tid] = x;
-      else dsmem_store(s_gat + rank * kRec + tid, 0, x);
+      else dsmem_store_f64(s_gat + rank * kRec + tid, 0, x);
     }
     team_sync();
     if (rank == 0 && warp == 0) {
@@ -1543,6 +1537,11 @@ int tile_trajectory_teams(int dp, int nstates) {
     case 128: return tile::teams_for<128>(nstates);
     default: return 0;
   }
+}
+
+int tile_trajectory_ctas(int dp, int nstates) {
+  const int teams = tile_trajectory_teams(dp, nstates), nb = dp <= 64 ? dp / 16 : dp / 32;
+  return nstates * teams * nb * nb;
 }
 
 cudaError_t tile_trajectory_launch(int dp, const TrajState* d_states, int nstates, const double* d_points, int npoints,

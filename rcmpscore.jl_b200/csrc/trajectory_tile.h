@@ -12,6 +12,7 @@ size_t tile_sync_bytes();                 // device bytes per state for the team
 // Teams (clusters of (dp/16)^2 CTAs up to dp = 64, (dp/32)^2 above) per state for a launch of nstates
 // states: 7, 4 or 2 when all teams of the launch are resident at once, else 1. 0: no cluster fits.
 int tile_trajectory_teams(int dp, int nstates);
+int tile_trajectory_ctas(int dp, int nstates);   // CTAs of that launch
 // The quartic trajectories of the states with herm set. zero_samples: also clear the structurally
 // zero sample tiles of packed Z2 states, which the kernel does not write.
 cudaError_t tile_trajectory_launch(int dp, const TrajState* d_states, int nstates, const double* d_points, int npoints,
