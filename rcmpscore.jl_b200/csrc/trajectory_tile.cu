@@ -129,6 +129,10 @@ template <int DP, bool LONE>
 struct Smem {
   using G = TG<DP>;
   static constexpr bool KSM = LONE && G::B == 16;       // stage vectors of the one owned tile
+  // a warp of its own for the other teams (B = 32 needs every register of the computing warps)
+  static constexpr bool COMM = LONE && G::B == 16;
+  static constexpr int IV = COMM ? G::BB : 0;
+  static constexpr int THREADS = G::NT + (COMM ? 32 : 0);
   static constexpr int KVEC = KSM ? 18 * G::BB : 0;
   static constexpr int XCH = G::NB == 1 ? 2 * (int)G::MAT : 0;   // X and P of a one-CTA team
   // the CTAs' records at rank 0, and the warps' error sums; at DP = 128 only a lone channel's fit
@@ -138,7 +142,7 @@ struct Smem {
   static constexpr int GAT = GLOBAL_REC ? 0 : G::NR * NREC / 2;
   static constexpr int WE = 2 * NC * G::NW / 2;
   static constexpr size_t bytes() {
-    return ((size_t)(G::PANEL + G::RJ) + G::RED + GAT + (GLOBAL_REC ? 0 : WE) + KVEC + XCH) * 16 + sizeof(Tail<G::NW>);
+    return ((size_t)(G::PANEL + G::RJ) + G::RED + GAT + (GLOBAL_REC ? 0 : WE) + KVEC + XCH + IV) * 16 + sizeof(Tail<G::NW>);
   }
 };
 
@@ -439,7 +443,7 @@ __device__ __forceinline__ double2 dense_value(const double2* cf, double2 yo, do
 }
 
 template <int DP, bool LONE>
-__global__ void __launch_bounds__(TG<DP>::NT, 1)
+__global__ void __launch_bounds__(Smem<DP, LONE>::THREADS, 1)
 tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ points, int npoints, TrajControls ctl_in,
             Sync* __restrict__ sync, int teams, int level) {
   using G = TG<DP>;
@@ -469,13 +473,18 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
   double* s_we = SM::GLOBAL_REC ? reinterpret_cast<double*>(s_red) : s_gat + 2 * SM::GAT;
   double2* s_k = s_red + G::RED + SM::GAT + (SM::GLOBAL_REC ? 0 : SM::WE);
   double2* s_x = s_k + SM::KVEC;
-  Tail<G::NW>& S = *reinterpret_cast<Tail<G::NW>*>(s_x + SM::XCH);
+  double2* s_iv = s_x + SM::XCH;                           // [BB] the insertion of the owned tile
+  Tail<G::NW>& S = *reinterpret_cast<Tail<G::NW>*>(s_iv + SM::IV);
   Ctl& C = S.ctl;
 
-  // the barrier of a team: a cluster barrier, or the block's own
+  // the barrier of a team: a cluster barrier, or the block's own; and the one of the warps that compute
   auto team_sync = [&]() {
     if constexpr (NR == 1) __syncthreads();
     else cluster_sync();
+  };
+  auto block_sync = [&]() {
+    if constexpr (SM::COMM) asm volatile("bar.sync 1, %0;" ::"n"(G::NT) : "memory");
+    else __syncthreads();
   };
   auto xload = [&](const double2* p) -> double2 {   // X and P of a team: L2, or shared memory when NB = 1
     if constexpr (NB == 1) return *p;
@@ -523,9 +532,9 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
   auto panel_of = [&](int dir) -> const double2* {
     if (!both) return s_panel;
     if (panel_dir != dir) {
-      __syncthreads();
+      block_sync();
       load_panel<DP>(st, dir, bi, s_panel);
-      __syncthreads();
+      block_sync();
       panel_dir = dir;
     }
     return s_panel;
@@ -533,9 +542,9 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
   auto rj_of = [&](int dir) -> const double2* {
     if (!both) return s_rj;
     if (rj_dir != dir) {
-      __syncthreads();
+      block_sync();
       load_rj<DP>(st, dir, bj, s_rj);
-      __syncthreads();
+      block_sync();
       rj_dir = dir;
     }
     return s_rj;
@@ -543,6 +552,55 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
 
   init_tail(S, G::NW, ctl_in.endpoint);
   __syncthreads();
+
+  if constexpr (SM::COMM) {
+    // The warp behind the computing ones talks to the other teams, so that no flag's or remote tile's
+    // round trip lies on their path: it takes part in every team barrier, brings the insertion of the
+    // owned tile to shared memory between the two barriers of a right-hand side, and flags the P tile
+    // after the second.
+    if (warp == G::NW) {
+      const int src = c_src[c0], dst = c_feeds[c0];
+      const bool takes = src >= 0 && owns(c0);
+      unsigned n = 0;
+      auto serve = [&]() {
+        ++n;
+        team_sync();
+        if (takes) {
+          if (lane == 0) {
+            flag_wait(&sy->pflag[src][rank], n, &S.wait_flag);
+            if (bi != bj) flag_wait(&sy->pflag[src][bj * NB + bi], n, &S.wait_flag);
+          }
+          __syncwarp();
+          const double2* ps = st->P + (size_t)(n & 15) * kChannels * MAT + (size_t)src * MAT;
+          double2 a[BB / 32], b[BB / 32];
+#pragma unroll
+          for (int q = 0; q < BB / 32; ++q) {   // element q * 32 + lane of the tile
+            const int r = 8 * ((q >> 1) & 1) + (lane >> 2), col = 8 * (q >> 2) + 2 * (lane & 3) + (q & 1);
+            a[q] = __ldcg(ps + poff<DP>(bi, bj, r, col));
+            b[q] = __ldcg(ps + poff<DP>(bj, bi, col, r));
+          }
+#pragma unroll
+          for (int q = 0; q < BB / 32; ++q) s_iv[q * 32 + lane] = zadd(a[q], zconj(b[q]));
+        }
+        team_sync();
+        if (dst >= 0 && lane == 0) {
+          __threadfence();
+          flag_release(&sy->pflag[c0][rank], n);
+        }
+      };
+      serve();
+      team_sync();
+      while (!S.dec.stop) {
+        for (int s = 1; s <= 12; ++s) serve();
+        team_sync();
+        team_sync();
+        if (S.dec.accept && S.dec.dense)
+          for (int s = 13; s < 16; ++s) serve();
+      }
+      team_sync();
+      return;
+    }
+  }
 
   int yslot = kSlotY, pslot = kSlotY + 1, k0slot = 0, k12slot = 12;
   auto kslot = [&](int s) { return s == 0 ? k0slot : s == 12 ? k12slot : s; };
@@ -620,12 +678,12 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         };
         if constexpr (G::FOLD) {
           if (sl >= G::SF1) deposit(sl - G::SF1, false);
-          __syncthreads();
+          block_sync();
           if (sl < G::SF1) deposit(sl, true);
         } else {
           deposit(sl, false);
         }
-        __syncthreads();
+        block_sync();
         if (owner_thread) {
           // sum of the partial tiles at (r, col) of row tile group mq (0: Y, 1: P)
           auto total = [&](int mq, int r, int col) {
@@ -662,9 +720,9 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
             }
           }
         }
-        if constexpr (!LONE) __syncthreads();
+        if constexpr (!LONE) block_sync();
       }
-      if (teams > 1) {
+      if (!SM::COMM && teams > 1) {
         // P tiles that another team inserts: complete, then flagged
         bool feeds = false;
         for (int c = c0; c < c1; ++c) {
@@ -672,7 +730,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
           feeds |= f >= 0 && (f < c0 || f >= c1);
         }
         if (feeds) {
-          __syncthreads();
+          block_sync();
           if (tid == 0) {
             __threadfence();
             for (int c = c0; c < c1; ++c) {
@@ -683,7 +741,22 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         }
       }
     }
-    team_sync();
+    if constexpr (SM::COMM || NR == 1) {
+      team_sync();
+    } else {
+      // the flags of the tiles that other teams insert are awaited while the barrier completes
+      cluster_arrive_release();
+      for (int c = c0; c < c1; ++c) {
+        const int s = c_src[c];
+        if (s < 0 || (s >= c0 && s < c1) || !owns(c)) continue;
+        if (lane == 0) {
+          flag_wait(&sy->pflag[s][rank], seq, &S.wait_flag);
+          if (bi != bj) flag_wait(&sy->pflag[s][bj * NB + bi], seq, &S.wait_flag);
+        }
+        __syncwarp();
+      }
+      cluster_wait_acquire();
+    }
     // ------------------------------------------------ phase 2
     {
       const int sl = warp / (G::MG2 * G::NG2), ng = warp % G::NG2, mg = (warp / G::NG2) % G::MG2;
@@ -705,7 +778,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         }
         // the epilogue's operands, in flight during the products (B = 32 loads them after: registers)
         const int s = c_src[c];
-        const bool remote = s >= 0 && (s < c0 || s >= c1);
+        const bool remote = !SM::COMM && s >= 0 && (s < c0 || s >= c1);
         const double2* ps = (remote ? st->P + (size_t)(seq & 15) * VEC : pw) + (size_t)(s >= 0 ? s : 0) * MAT;
         const double2* fx = c == 0 ? st->fixed0 : c == 6 ? st->fixed6 : nullptr;
         double2 ev[EPT], iv[EPT];   // Y's other half, the insertion P_s + P_s^dag
@@ -720,20 +793,15 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
           }
           ev[it] = v;
           v = make_double2(0.0, 0.0);
-          if (s >= 0) {
+          if (SM::COMM) {
+            if (s >= 0) v = s_iv[e];
+          } else if (s >= 0) {
             const double2 *p1 = ps + poff<DP>(bi, bj, r, col), *p2 = ps + poff<DP>(bj, bi, col, r);
             const double2 a = remote ? __ldcg(p1) : xload(p1), b = remote ? __ldcg(p2) : xload(p2);
             v = zadd(a, zconj(b));
           }
           iv[it] = v;
         };
-        if (remote) {
-          if (lane == 0) {
-            flag_wait(&sy->pflag[s][rank], seq, &S.wait_flag);
-            if (bi != bj) flag_wait(&sy->pflag[s][bj * NB + bi], seq, &S.wait_flag);
-          }
-          __syncwarp();
-        }
         if (B == 16 && owner_thread) {
 #pragma unroll
           for (int it = 0; it < EPT; ++it) operands(it);
@@ -777,12 +845,12 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         };
         if constexpr (G::FOLD) {
           if (sl >= G::SF2) deposit(sl - G::SF2, false);
-          __syncthreads();
+          block_sync();
           if (sl < G::SF2) deposit(sl, true);
         } else {
           if (works) deposit(sl, false);
         }
-        __syncthreads();
+        block_sync();
         if (owner_thread) {
           if (B == 32) {
 #pragma unroll
@@ -804,7 +872,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
             kout[e] = v;
           }
         }
-        if constexpr (!LONE) __syncthreads();
+        if constexpr (!LONE) block_sync();
       }
     }
   };
@@ -841,9 +909,9 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
   while (!stop) {
     ++attempt;
     const double t = S.dec.nt, h = S.dec.nh;
-    __syncthreads();
+    block_sync();
     stage_times(S, t, h);
-    __syncthreads();
+    block_sync();
     // ------------------------------------------------------------ stages 1..12
     for (int s = 1; s <= 12; ++s) {
       const double* w = s == 12 ? c_dop_b : c_dop_a + 16 * s;
@@ -877,7 +945,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
       rhs(kslot(s), S.jac[s], S.src[s]);
     }
     // ------------------------------------------------------------ error norms
-    if constexpr (SM::GLOBAL_REC) __syncthreads();   // the last stage's partial tiles have been read
+    if constexpr (SM::GLOBAL_REC) block_sync();   // the last stage's partial tiles have been read
     for (int c = c0; c < c1; ++c) {
       double s5 = 0.0, s3 = 0.0;
       if (owns(c) && owner_thread) {
@@ -910,7 +978,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         s_we[(SM::NC + (LONE ? 0 : c)) * G::NW + warp] = s3;
       }
     }
-    __syncthreads();
+    block_sync();
     // the CTA's record (kRec; a lone channel's: both error sums, then 14..19) into rank 0
     if (tid < SM::NREC) {
       const int v = !LONE ? tid : tid < 2 ? 7 * tid + c0 : tid + 12;
@@ -1476,7 +1544,7 @@ template <int DP>
 static int teams_for(int nstates) {
   using G = TG<DP>;
   static_assert(Smem<DP, true>::bytes() <= 232448, "shared memory per CTA");
-  if ((long long)nstates * 7 <= resident_clusters<DP>(tile_kernel<DP, true>, G::NT, Smem<DP, true>::bytes())) return 7;
+  if ((long long)nstates * 7 <= resident_clusters<DP>(tile_kernel<DP, true>, Smem<DP, true>::THREADS, Smem<DP, true>::bytes())) return 7;
   if constexpr (G::B == 16) {
     return resident_clusters<DP>(wide_kernel<DP>, Wide<DP>::NT, Wide<DP>::BYTES) >= 1 ? 1 : 0;
   } else {
@@ -1502,7 +1570,8 @@ static cudaError_t launch(const TrajState* d_states, int nstates, const double* 
   }
   note_launch();
   if (teams == 7) {
-    e = configure<DP>(tile_kernel<DP, true>, nstates * teams, G::NT, Smem<DP, true>::bytes(), true, stream, attr, cfg);
+    e = configure<DP>(tile_kernel<DP, true>, nstates * teams, Smem<DP, true>::THREADS, Smem<DP, true>::bytes(), true, stream,
+                      attr, cfg);
     if (e != cudaSuccess) return e;
     return cudaLaunchKernelEx(&cfg, tile_kernel<DP, true>, d_states, d_points, npoints, ctl, (Sync*)sync, teams, level);
   }
