@@ -36,7 +36,7 @@ constexpr int kNodesPerBlock = 32;
 
 // Per-system sizes: channels of a stage vector, operator matrices, stage vectors of the
 // trajectory workspace (k[18], the last two of them y and prop, z[2], P, and L for the all-ODE
-// route; the quartic system's tile kernel has z[3] and P[16]), pullback scratch, partial and
+// route; the quartic system's tile kernels have two partial sums behind k[18], z[3] and P[16]), pullback scratch, partial and
 // finalize matrices per state.
 struct SysSizes {
   int nch, nops, nwork;
@@ -47,7 +47,7 @@ SysSizes sys_sizes(int system, int dp, int nblk) {
   z.nch = trajectory_channels(system);
   if (system == 0) {
     z.nops = kOps;
-    z.nwork = 37;
+    z.nwork = 39;
     z.wscr = (size_t)nblk * pullback_row_blocks(dp) * 3;
     z.part = (size_t)nblk * 4;
     z.fin = 8;
@@ -297,8 +297,8 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
         t.k = w;
         t.y = w + 16 * vec;
         t.prop = w + 17 * vec;
-        t.z = w + 18 * vec;
-        t.P = w + (system == 0 ? 21 : 20) * vec;
+        t.z = w + (system == 0 ? 20 : 18) * vec;
+        t.P = w + (system == 0 ? 23 : 20) * vec;
         t.L = system == 1 ? w + 21 * vec : nullptr;
         t.samples = d_samp + (size_t)i * npoints * vec;
         t.stats = reinterpret_cast<TrajStats*>(base + o_tstats) + i;

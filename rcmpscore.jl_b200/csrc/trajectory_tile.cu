@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 #include "common.cuh"
 #include "dop853_device.cuh"
 #include "trajectory.h"
@@ -174,9 +175,16 @@ __device__ __forceinline__ size_t poff(int a, int b, int r, int c) {
   return ((size_t)(a * G::KS + b * G::KB + c / 8) * G::MT + r / 16) * 128 + (((r >> 3) & 1) + 2 * ((c >> 2) & 1)) * 32 +
          4 * (r & 7) + (c & 3);
 }
-// Entry (r, c) of a 16 x 8 tile in C-fragment order [4][32].
+// Entry (r, c) of a 16 x 8 tile in C-fragment order [4][32]; and its place in a partial tile in shared
+// memory, where the lanes are permuted so that a warp reads a tile's entries and their mirrors without
+// bank conflicts (unpermuted, the mirrors met 8-way).
 __device__ __forceinline__ int roff(int r, int c) {
   return (2 * ((r >> 3) & 1) + (c & 1)) * 32 + 4 * (r & 7) + ((c & 7) >> 1);
+}
+
+__device__ __forceinline__ int swz(int i, int lane) { return i * 32 + (lane ^ ((lane >> 3) & 3) ^ (4 * (i & 1))); }
+__device__ __forceinline__ int soff(int r, int c) {
+  return swz(2 * ((r >> 3) & 1) + (c & 1), 4 * (r & 7) + ((c & 7) >> 1));
 }
 
 // The CTA's [Qc; Rc] rows of block bi as A fragments [KS][2 MT][4][32], and the columns bj of Rc^dag as
@@ -566,10 +574,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         ++n;
         team_sync();
         if (takes) {
-          if (lane == 0) {
-            flag_wait(&sy->pflag[src][rank], n, &S.wait_flag);
-            if (bi != bj) flag_wait(&sy->pflag[src][bj * NB + bi], n, &S.wait_flag);
-          }
+          if (lane < 2) flag_wait(&sy->pflag[src][lane ? bj * NB + bi : rank], n, &S.wait_flag);
           __syncwarp();
           const double2* ps = st->P + (size_t)(n & 15) * kChannels * MAT + (size_t)src * MAT;
           double2 a[BB / 32], b[BB / 32];
@@ -608,10 +613,17 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
   double2 yown[LONE ? EPT : 1];          // Y(i, j) (+ its mirror on the diagonal) of the one owned channel
 
   // ---------------------------------------------------------------- one right-hand side
-  // X_c of the team's channels is in gz; k of the owned tiles goes to slot ks_out.
-  auto rhs = [&](int ks_out, double jac, double src) {
+  // X_c of the team's channels is in gz; k of the owned tiles goes to slot ks_out. during(): work on the
+  // thread's own stage vectors, done while the team's barrier completes.
+  auto rhs = [&](int ks_out, double jac, double src, auto&& during) {
     ++seq;
-    team_sync();
+    if constexpr (NR == 1 || B == 32) {
+      team_sync();
+    } else {
+      cluster_arrive_release();
+      during();
+      cluster_wait_acquire();
+    }
     double2* const pw = gp + (size_t)(seq & 15) * pstep;
     // ------------------------------------------------ phase 1
     {
@@ -671,9 +683,9 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         auto deposit = [&](int slot, bool add) {
 #pragma unroll
           for (int m = 0; m < G::M1; ++m) {
-            double2* p = red + ((size_t)slot * G::T1 + (mg * G::M1 + m) * NTB + nt) * 128 + lane;
+            double2* p = red + ((size_t)slot * G::T1 + (mg * G::M1 + m) * NTB + nt) * 128;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) p[32 * i] = add ? zadd(p[32 * i], acc[m].value(i)) : acc[m].value(i);
+            for (int i = 0; i < 4; ++i) p[swz(i, lane)] = add ? zadd(p[swz(i, lane)], acc[m].value(i)) : acc[m].value(i);
           }
         };
         if constexpr (G::FOLD) {
@@ -687,7 +699,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         if (owner_thread) {
           // sum of the partial tiles at (r, col) of row tile group mq (0: Y, 1: P)
           auto total = [&](int mq, int r, int col) {
-            const double2* p = red + ((size_t)(mq * MT + r / 16) * NTB + col / 8) * 128 + roff(r, col);
+            const double2* p = red + ((size_t)(mq * MT + r / 16) * NTB + col / 8) * 128 + soff(r, col);
             double2 v = p[0];
 #pragma unroll
             for (int s = 1; s < G::SF1; ++s) v = zadd(v, p[(size_t)s * G::T1 * 128]);
@@ -741,18 +753,17 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         }
       }
     }
+    if constexpr (NR == 1) during();
     if constexpr (SM::COMM || NR == 1) {
       team_sync();
     } else {
       // the flags of the tiles that other teams insert are awaited while the barrier completes
       cluster_arrive_release();
+      if constexpr (B == 32) during();   // the owners are the last at the first barrier
       for (int c = c0; c < c1; ++c) {
         const int s = c_src[c];
         if (s < 0 || (s >= c0 && s < c1) || !owns(c)) continue;
-        if (lane == 0) {
-          flag_wait(&sy->pflag[s][rank], seq, &S.wait_flag);
-          if (bi != bj) flag_wait(&sy->pflag[s][bj * NB + bi], seq, &S.wait_flag);
-        }
+        if (lane < 2) flag_wait(&sy->pflag[s][lane ? bj * NB + bi : rank], seq, &S.wait_flag);
         __syncwarp();
       }
       cluster_wait_acquire();
@@ -838,9 +849,9 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         auto deposit = [&](int slot, bool add) {
 #pragma unroll
           for (int n = 0; n < G::N2; ++n) {
-            double2* p = red + ((size_t)slot * G::T2 + mg * NTB + ng * G::N2 + n) * 128 + lane;
+            double2* p = red + ((size_t)slot * G::T2 + mg * NTB + ng * G::N2 + n) * 128;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) p[32 * i] = add ? zadd(p[32 * i], acc[n].value(i)) : acc[n].value(i);
+            for (int i = 0; i < 4; ++i) p[swz(i, lane)] = add ? zadd(p[swz(i, lane)], acc[n].value(i)) : acc[n].value(i);
           }
         };
         if constexpr (G::FOLD) {
@@ -861,7 +872,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
           for (int it = 0; it < EPT; ++it) {
             const int e = it * G::OWN + tid, r = el_r(it), col = el_c(it);
             if (!el_active(r, col)) continue;
-            const double2* p = red + ((size_t)(r / 16) * NTB + col / 8) * 128 + roff(r, col);
+            const double2* p = red + ((size_t)(r / 16) * NTB + col / 8) * 128 + soff(r, col);
             double2 v = p[0];
 #pragma unroll
             for (int q = 1; q < G::SF2; ++q) v = zadd(v, p[(size_t)q * G::T2 * 128]);
@@ -884,6 +895,71 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
     if (bi != bj || r != col) z[zoff<DP>(bj, bi, col, r)] = zconj(v);
   };
 
+  // Of a stage vector y + h sum_j w_j k_j only the last term waits for the right-hand side before it: the
+  // others are summed during that right-hand side, in the same order (a register, or slots 18 and 19).
+  // At DP = 128 the stage vectors' loads are the owners' critical path either way and the detour
+  // through a slot costs more than the wait hides (Z2 D = 128 16.0 -> 18.2 us, D = 64 6.8 -> 6.1):
+  // there the sum is taken when it is used.
+  constexpr bool EARLY = DP != 128;
+  constexpr int kSlotSum = 18;
+  double2 psum[2];
+  auto sum_put = [&](int q, int c, int it, double2 v) {
+    if constexpr (SM::KSM) psum[q] = v;
+    else kvec(kSlotSum + q, c)[it * G::OWN + tid] = v;
+  };
+  auto sum_get = [&](int q, int c, int it) -> double2 {
+    if constexpr (SM::KSM) return psum[q];
+    else return kvec(kSlotSum + q, c)[it * G::OWN + tid];
+  };
+  // y + the first n terms of the weights w (at most MAX) of one entry
+  auto entry_sum = [&](const double* w, int n, double h, auto max, int c, int it) -> double2 {
+    constexpr int MAX = decltype(max)::value;
+    const int e = it * G::OWN + tid;
+    double2 kv[MAX];
+#pragma unroll
+    for (int j = 0; j < MAX; ++j)
+      kv[j] = j < n && w[j] != 0.0 ? kvec(kslot(j), c)[e] : make_double2(0.0, 0.0);
+    double2 v = kvec(yslot, c)[e];
+#pragma unroll
+    for (int j = 0; j < MAX; ++j) v = zaxpy(j < n ? h * w[j] : 0.0, kv[j], v);
+    return v;
+  };
+  // both error estimates of one entry without k_12
+  auto entry_errors = [&](int c, int it, double2& e5, double2& e3) {
+    double2 kv[12];
+#pragma unroll
+    for (int j = 0; j < 12; ++j) kv[j] = kvec(kslot(j), c)[it * G::OWN + tid];
+    e5 = e3 = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int j = 0; j < 12; ++j) {
+      e5 = zaxpy(c_dop_e5[j], kv[j], e5);
+      e3 = zaxpy(c_dop_e3[j], kv[j], e3);
+    }
+  };
+  auto partial_sum = [&](const double* w, int n, double h, auto max) {
+    if constexpr (EARLY) {
+      for (int c = c0; c < c1; ++c) {
+        if (!owns(c) || !owner_thread) continue;
+#pragma unroll
+        for (int it = 0; it < EPT; ++it) sum_put(0, c, it, entry_sum(w, n, h, max, c, it));
+      }
+    }
+  };
+  auto partial_errors = [&]() {
+    if constexpr (EARLY) {
+      for (int c = c0; c < c1; ++c) {
+        if (!owns(c) || !owner_thread) continue;
+#pragma unroll
+        for (int it = 0; it < EPT; ++it) {
+          double2 e5, e3;
+          entry_errors(c, it, e5, e3);
+          sum_put(0, c, it, e5);
+          sum_put(1, c, it, e3);
+        }
+      }
+    }
+  };
+
   // ---------------------------------------------------------------- start: y = 0, k0 = f(-a, 0)
   for (int c = c0; c < c1; ++c) {
     if (!owns(c) || !owner_thread) continue;
@@ -896,7 +972,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
       put_z(c, it, r, col, z0);
     }
   }
-  rhs(k0slot, S.jac[0], S.src[0]);
+  rhs(k0slot, S.jac[0], S.src[0], [] {});
 
   const double atol = st->atol, rtol = st->rtol;
   const double N = packed ? 10.0 * half * half + 1.0 : (double)kChannels * st->d * st->d + 1.0;
@@ -918,18 +994,14 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
       double part = 0.0;
       for (int c = c0; c < c1; ++c) {
         if (!owns(c) || !owner_thread) continue;
-        const double2* yv = kvec(yslot, c);
 #pragma unroll
         for (int it = 0; it < EPT; ++it) {
           const int e = it * G::OWN + tid, r = el_r(it), col = el_c(it);
           if (!el_active(r, col)) continue;
-          double2 kv[12];
-#pragma unroll
-          for (int j = 0; j < 12; ++j)
-            kv[j] = j < s && w[j] != 0.0 ? kvec(kslot(j), c)[e] : make_double2(0.0, 0.0);
-          double2 v = yv[e];
-#pragma unroll
-          for (int j = 0; j < 12; ++j) v = zaxpy(j < s ? h * w[j] : 0.0, kv[j], v);
+          double2 base;
+          if constexpr (EARLY) base = s == 1 ? kvec(yslot, c)[e] : sum_get(0, c, it);
+          else base = entry_sum(w, s - 1, h, std::integral_constant<int, 11>(), c, it);
+          const double2 v = zaxpy(h * w[s - 1], kvec(kslot(s - 1), c)[e], base);
           put_z(c, it, r, col, v);
           if (s == 12) kvec(pslot, c)[e] = v;
           if (c == 2) {
@@ -942,7 +1014,10 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         part = warp_sum(part);
         if (lane == 0) S.wk[s][warp] = part;
       }
-      rhs(kslot(s), S.jac[s], S.src[s]);
+      rhs(kslot(s), S.jac[s], S.src[s], [&] {
+        if (s < 12) partial_sum(s == 11 ? c_dop_b : c_dop_a + 16 * (s + 1), s, h, std::integral_constant<int, 11>());
+        else partial_errors();
+      });
     }
     // ------------------------------------------------------------ error norms
     if constexpr (SM::GLOBAL_REC) block_sync();   // the last stage's partial tiles have been read
@@ -956,15 +1031,16 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         const int row = bi * B + r, cl = bj * B + col;
         const double wt = norm_weight(packed, half, c, row, cl);
         if (wt == 0.0) continue;
-        double2 kv[13];
-#pragma unroll
-        for (int j = 0; j <= 12; ++j) kv[j] = kvec(kslot(j), c)[e];
-        double2 e5 = make_double2(0.0, 0.0), e3 = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int j = 0; j <= 12; ++j) {
-          e5 = zaxpy(c_dop_e5[j], kv[j], e5);
-          e3 = zaxpy(c_dop_e3[j], kv[j], e3);
+        const double2 k12 = kvec(kslot(12), c)[e];
+        double2 e5, e3;
+        if constexpr (EARLY) {
+          e5 = sum_get(0, c, it);
+          e3 = sum_get(1, c, it);
+        } else {
+          entry_errors(c, it, e5, e3);
         }
+        e5 = zaxpy(c_dop_e5[12], k12, e5);
+        e3 = zaxpy(c_dop_e3[12], k12, e3);
         const double2 yo = kvec(yslot, c)[e], yn = kvec(pslot, c)[e];
         const double scale = atol + rtol * fmax(hypot(yo.x, yo.y), hypot(yn.x, yn.y));
         s5 += wt * (zabs2(e5) / (scale * scale));
@@ -1022,25 +1098,23 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
     if (S.dec.accept) {
       if (S.dec.dense) {
         // dense stages 13..15
+        partial_sum(c_dop_a + 16 * 13, 12, h, std::integral_constant<int, 12>());
         for (int s = 13; s < 16; ++s) {
           for (int c = c0; c < c1; ++c) {
             if (!owns(c) || !owner_thread) continue;
-            const double2* yv = kvec(yslot, c);
 #pragma unroll
             for (int it = 0; it < EPT; ++it) {
               const int e = it * G::OWN + tid, r = el_r(it), col = el_c(it);
               if (!el_active(r, col)) continue;
-              double2 kv[15];
-#pragma unroll
-              for (int j = 0; j < 15; ++j)
-                kv[j] = j < s && c_dop_a[16 * s + j] != 0.0 ? kvec(kslot(j), c)[e] : make_double2(0.0, 0.0);
-              double2 v = yv[e];
-#pragma unroll
-              for (int j = 0; j < 15; ++j) v = zaxpy(j < s ? h * c_dop_a[16 * s + j] : 0.0, kv[j], v);
-              put_z(c, it, r, col, v);
+              double2 base;
+              if constexpr (EARLY) base = sum_get(0, c, it);
+              else base = entry_sum(c_dop_a + 16 * s, s - 1, h, std::integral_constant<int, 14>(), c, it);
+              put_z(c, it, r, col, zaxpy(h * c_dop_a[16 * s + s - 1], kvec(kslot(s - 1), c)[e], base));
             }
           }
-          rhs(s, S.jac[s], S.src[s]);
+          rhs(s, S.jac[s], S.src[s], [&] {
+            if (s < 15) partial_sum(c_dop_a + 16 * (s + 1), s, h, std::integral_constant<int, 14>());
+          });
         }
         // order-7 interpolation at the nodes in (t, t_new]
         const double tn = S.dec.tn;
@@ -1222,10 +1296,17 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
     }
   };
 
-  auto rhs = [&](int ks_out, double jac, double src) {
+  auto rhs = [&](int ks_out, double jac, double src, auto&& during) {   // during(): as in tile_kernel
     ++seq;
-    if constexpr (NB > 1) fence_proxy_async_global();
-    team_sync();
+    if constexpr (NR == 1) {
+      during();
+      team_sync();
+    } else {
+      fence_proxy_async_global();
+      cluster_arrive_release();
+      during();
+      cluster_wait_acquire();
+    }
     if (NB > 1 && tid == 0) {
       fence_proxy_async_global();
       fence_proxy_async_shared();
@@ -1312,6 +1393,45 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
     if (bi != bj || r != col) z[zoff<DP>(bj, bi, col, r)] = zconj(v);
   };
 
+  // partial sums of the next stage vector and of the error estimates, in slots 18 and 19 (tile_kernel)
+  auto partial_sum = [&](const double* w, int n, double h, auto max) {
+    constexpr int MAX = decltype(max)::value;
+    if (!own) return;
+#pragma unroll
+    for (int it = 0; it < NPT; ++it)
+#pragma unroll 2
+      for (int i = 0; i < 4; ++i) {
+        const int e = el_e(nt0 + it, i);
+        double2 kv[MAX];
+#pragma unroll
+        for (int j = 0; j < MAX; ++j) kv[j] = j < n && w[j] != 0.0 ? kvec(kslot(j))[e] : make_double2(0.0, 0.0);
+        double2 v = kvec(yslot)[e];
+#pragma unroll
+        for (int j = 0; j < MAX; ++j) v = zaxpy(j < n ? h * w[j] : 0.0, kv[j], v);
+        kvec(18)[e] = v;
+      }
+  };
+  auto partial_errors = [&]() {
+    if (!own) return;
+#pragma unroll
+    for (int it = 0; it < NPT; ++it)
+#pragma unroll 1
+      for (int i = 0; i < 4; ++i) {
+        const int e = el_e(nt0 + it, i);
+        double2 kv[12];
+#pragma unroll
+        for (int j = 0; j < 12; ++j) kv[j] = kvec(kslot(j))[e];
+        double2 e5 = make_double2(0.0, 0.0), e3 = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int j = 0; j < 12; ++j) {
+          e5 = zaxpy(c_dop_e5[j], kv[j], e5);
+          e3 = zaxpy(c_dop_e3[j], kv[j], e3);
+        }
+        kvec(18)[e] = e5;
+        kvec(19)[e] = e3;
+      }
+  };
+
   // ---------------------------------------------------------------- start: y = 0, k0 = f(-a, 0)
   if (own) {
 #pragma unroll
@@ -1324,7 +1444,7 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         put_z(r, col, make_double2(0.0, 0.0));
       }
   }
-  rhs(k0slot, S.jac[0], S.src[0]);
+  rhs(k0slot, S.jac[0], S.src[0], [] {});
 
   const double atol = st->atol, rtol = st->rtol;
   const double N = packed ? 10.0 * half * half + 1.0 : (double)kChannels * st->d * st->d + 1.0;
@@ -1343,18 +1463,12 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
       if (own) {
 #pragma unroll
         for (int it = 0; it < NPT; ++it)
-#pragma unroll 2
+#pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int nt = nt0 + it, r = el_r(i), col = el_c(nt, i), e = el_e(nt, i);
             double part = 0.0;
             if (active(r, col)) {
-              double2 kv[12];
-#pragma unroll
-              for (int j = 0; j < 12; ++j)
-                kv[j] = j < s && w[j] != 0.0 ? kvec(kslot(j))[e] : make_double2(0.0, 0.0);
-              double2 v = kvec(yslot)[e];
-#pragma unroll
-              for (int j = 0; j < 12; ++j) v = zaxpy(j < s ? h * w[j] : 0.0, kv[j], v);
+              const double2 v = zaxpy(h * w[s - 1], kvec(kslot(s - 1))[e], kvec(s == 1 ? yslot : 18)[e]);
               put_z(r, col, v);
               if (s == 12) kvec(pslot)[e] = v;
               if (c == 2) {
@@ -1368,7 +1482,10 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
             }
           }
       }
-      rhs(kslot(s), S.jac[s], S.src[s]);
+      rhs(kslot(s), S.jac[s], S.src[s], [&] {
+        if (s < 12) partial_sum(s == 11 ? c_dop_b : c_dop_a + 16 * (s + 1), s, h, std::integral_constant<int, 11>());
+        else partial_errors();
+      });
     }
     // ------------------------------------------------------------ error norms
     if (own) {
@@ -1380,15 +1497,8 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
           double s5 = 0.0, s3 = 0.0;
           const double wt = active(r, col) ? norm_weight(packed, half, c, bi * B + r, bj * B + col) : 0.0;
           if (wt != 0.0) {
-            double2 kv[13];
-#pragma unroll
-            for (int j = 0; j <= 12; ++j) kv[j] = kvec(kslot(j))[e];
-            double2 e5 = make_double2(0.0, 0.0), e3 = make_double2(0.0, 0.0);
-#pragma unroll
-            for (int j = 0; j <= 12; ++j) {
-              e5 = zaxpy(c_dop_e5[j], kv[j], e5);
-              e3 = zaxpy(c_dop_e3[j], kv[j], e3);
-            }
+            const double2 k12 = kvec(kslot(12))[e];
+            const double2 e5 = zaxpy(c_dop_e5[12], k12, kvec(18)[e]), e3 = zaxpy(c_dop_e3[12], k12, kvec(19)[e]);
             const double2 yo = kvec(yslot)[e], yn = kvec(pslot)[e];
             const double scale = atol + rtol * fmax(hypot(yo.x, yo.y), hypot(yn.x, yn.y));
             s5 += wt * (zabs2(e5) / (scale * scale));
@@ -1424,25 +1534,21 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
     stop = S.dec.stop != 0;
     if (S.dec.accept) {
       if (S.dec.dense) {
+        partial_sum(c_dop_a + 16 * 13, 12, h, std::integral_constant<int, 12>());
         for (int s = 13; s < 16; ++s) {
           if (own) {
 #pragma unroll
             for (int it = 0; it < NPT; ++it)
-#pragma unroll 1
+#pragma unroll
               for (int i = 0; i < 4; ++i) {
                 const int nt = nt0 + it, r = el_r(i), col = el_c(nt, i), e = el_e(nt, i);
                 if (!active(r, col)) continue;
-                double2 kv[15];
-#pragma unroll
-                for (int j = 0; j < 15; ++j)
-                  kv[j] = j < s && c_dop_a[16 * s + j] != 0.0 ? kvec(kslot(j))[e] : make_double2(0.0, 0.0);
-                double2 v = kvec(yslot)[e];
-#pragma unroll
-                for (int j = 0; j < 15; ++j) v = zaxpy(j < s ? h * c_dop_a[16 * s + j] : 0.0, kv[j], v);
-                put_z(r, col, v);
+                put_z(r, col, zaxpy(h * c_dop_a[16 * s + s - 1], kvec(kslot(s - 1))[e], kvec(18)[e]));
               }
           }
-          rhs(s, S.jac[s], S.src[s]);
+          rhs(s, S.jac[s], S.src[s], [&] {
+            if (s < 15) partial_sum(c_dop_a + 16 * (s + 1), s, h, std::integral_constant<int, 14>());
+          });
         }
         const double tn = S.dec.tn;
         const long long first = S.dec.first, last = S.dec.last;
