@@ -36,7 +36,7 @@ constexpr int kNodesPerBlock = 32;
 
 // Per-system sizes: channels of a stage vector, operator matrices, stage vectors of the
 // trajectory workspace (k[18], the last two of them y and prop, z[2], P, and L for the all-ODE
-// route; the quartic system's tile kernels have two partial sums behind k[18], z[3] and P[16]), pullback scratch, partial and
+// route; the quartic system's tile kernels have two partial sums behind k[18], z[3] and P[32]), pullback scratch, partial and
 // finalize matrices per state.
 struct SysSizes {
   int nch, nops, nwork;
@@ -47,7 +47,7 @@ SysSizes sys_sizes(int system, int dp, int nblk) {
   z.nch = trajectory_channels(system);
   if (system == 0) {
     z.nops = kOps;
-    z.nwork = 39;
+    z.nwork = 55;
     z.wscr = (size_t)nblk * pullback_row_blocks(dp) * 3;
     z.part = (size_t)nblk * 4;
     z.fin = 8;

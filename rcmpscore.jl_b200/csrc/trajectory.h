@@ -24,7 +24,7 @@ struct TrajState {
   const double2* rho;                 // initial value of the rho channels (all-ODE route)
   double2 *y, *prop, *k, *z, *P;      // y, proposed [V]; k [16][V]; z [2][V]; P [V]; V = channels dp^2
                                       // (quartic system: k [20][V], y and prop its slots 16 and 17, z [3][V],
-                                      // P [16][V], as the tile kernels use them)
+                                      // P [32][V], as the tile kernels use them)
   double2* L;                         // [V] commutator products O X (all-ODE route)
   double2* samples;                   // [npoints][V]
   TrajStats* stats;

@@ -107,7 +107,8 @@ struct TG {
 struct Dec {
   double t, h, tn;            // the attempt just judged
   double nt, nh;              // the next attempt
-  int accept, dense, stop, pad;
+  int accept, dense, stop;
+  int spec;                   // the next attempt has sample points in its step: its dense stages are due if accepted
   long long first, last;
 };
 struct Ctl {
@@ -229,7 +230,14 @@ __device__ __forceinline__ void prepare_attempt(double t, double h0, double endp
   else if (!isfinite(h) || h <= 10.0 * fabs(next_up(t) - t)) status = kStepUnderflow;
 }
 
-// Rank 0's warp 0 hands a decision to every CTA of the team.
+// Whether an attempt from t with step h would step over the sample point `next`.
+__device__ __forceinline__ int has_points(double t, double h, double endpoint, const double* points, long long next,
+                                          int npoints) {
+  const double boundary = t < 0.0 ? 0.0 : endpoint;
+  return next < npoints && points[next] <= (h == boundary - t ? boundary : __dadd_rn(t, h));
+}
+
+// A warp of rank 0 hands a decision to every CTA of the team.
 template <int NR>
 __device__ __forceinline__ void share_dec(Dec* shared, const Dec& d) {
   const int lane = threadIdx.x & 31;
@@ -245,12 +253,14 @@ __device__ __forceinline__ void share_dec(Dec* shared, const Dec& d) {
 
 // The first decision of a trajectory (rank 0's warp 0).
 template <int NR, class TailT>
-__device__ void first_decision(TailT& S, const TrajState* st, const TrajControls& ctl) {
+__device__ void first_decision(TailT& S, const TrajState* st, const TrajControls& ctl, const double* points,
+                               int npoints) {
   Dec d{};
   int status = 0;
   d.nt = -ctl.endpoint;
   prepare_attempt(d.nt, fmin(ctl.initial_h, 2.0 * ctl.endpoint), ctl.endpoint, 0, st->max_steps, d.nh, status);
   d.stop = status ? 1 : 0;
+  d.spec = has_points(d.nt, d.nh, ctl.endpoint, points, 0, npoints);
   if ((threadIdx.x & 31) == 0) {
     S.ctl.status = status;
     if (!status) {
@@ -263,7 +273,7 @@ __device__ void first_decision(TailT& S, const TrajState* st, const TrajControls
 }
 
 // The controller (ode_backend.py:529-547; persistent_trajectory_backend.py:109-131) on the state's
-// record in S.tot, by rank 0's warp 0, every lane alike; pt: the lane's next sample point.
+// record in S.tot, by one warp of rank 0, every lane alike; pt: the lane's next sample point.
 template <int NR, class TailT>
 __device__ void decide(TailT& S, const TrajState* st, const TrajControls& ctl, const double* points, int npoints,
                        double pt, double N, double t, double h) {
@@ -331,6 +341,7 @@ __device__ void decide(TailT& S, const TrajState* st, const TrajControls& ctl, c
       prepare_attempt(d.nt, hn, ctl.endpoint, C.attempts, st->max_steps, d.nh, status);
   }
   d.stop = status || d.nt >= ctl.endpoint ? 1 : 0;
+  if (!d.stop) d.spec = has_points(d.nt, d.nh, ctl.endpoint, points, np, npoints);
   __syncwarp();
   if (lane == 0) {
     C.err = err;
@@ -561,22 +572,61 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
   init_tail(S, G::NW, ctl_in.endpoint);
   __syncthreads();
 
+  // The exchange of the records, by one warp of rank 0. post: lane v sums entry v over the team's CTAs
+  // and publishes it; collect: the sum over the teams, and the decision on the attempt (t, h).
+  const double N = packed ? 10.0 * half * half + 1.0 : (double)kChannels * st->d * st->d + 1.0;
+  double team_tot = 0.0;
+  auto post = [&](unsigned attempt) {
+    const int own = !LONE ? lane : lane >= 14 ? lane - 12 : lane == c0 ? 0 : lane == 7 + c0 ? 1 : -1;
+    team_tot = 0.0;
+    if (lane < kRec && own >= 0)
+      for (int g = 0; g < NR; ++g)
+        team_tot += SM::GLOBAL_REC ? __ldcg(&sy->crec[team][g][own]) : s_gat[SM::NREC * g + own];
+    if (teams > 1) {
+      if (lane < kRec) sy->rec[team][attempt & 1][lane] = team_tot;
+      __syncwarp();
+      if (lane == 0) {
+        __threadfence();
+        flag_release(&sy->rflag[team], attempt);
+      }
+    }
+  };
+  auto collect = [&](unsigned attempt, double t, double h) {
+    const long long next = C.next_point;
+    const double pt = next + lane < npoints ? points[next + lane] : INFINITY;
+    double tot = team_tot;
+    if (teams > 1) {
+      if (lane < teams) flag_wait(&sy->rflag[lane], attempt, &S.wait_flag);
+      __syncwarp();
+      tot = 0.0;
+      if (lane < kRec)
+        for (int g = 0; g < teams; ++g) tot += __ldcg(&sy->rec[g][attempt & 1][lane]);
+      if (lane == 18 && S.wait_flag) tot = 1.0;
+    }
+    if (lane < kRec) S.tot[lane] = tot;
+    __syncwarp();
+    decide<NR>(S, st, ctl_in, points, npoints, pt, N, t, h);
+  };
+
   if constexpr (SM::COMM) {
     // The warp behind the computing ones talks to the other teams, so that no flag's or remote tile's
     // round trip lies on their path: it takes part in every team barrier, brings the insertion of the
     // owned tile to shared memory between the two barriers of a right-hand side, and flags the P tile
-    // after the second.
+    // after the second. Rank 0's also exchanges the records and decides on the attempt: while the
+    // other warps go on with the dense stages when the step holds sample points (they are due unless
+    // the attempt is rejected, one in twenty or fewer), so the exchange, 7 to 15 us, is off the path.
     if (warp == G::NW) {
       const int src = c_src[c0], dst = c_feeds[c0];
       const bool takes = src >= 0 && owns(c0);
       unsigned n = 0;
-      auto serve = [&]() {
+      auto serve = [&](auto&& after) {
         ++n;
         team_sync();
+        after();
         if (takes) {
           if (lane < 2) flag_wait(&sy->pflag[src][lane ? bj * NB + bi : rank], n, &S.wait_flag);
           __syncwarp();
-          const double2* ps = st->P + (size_t)(n & 15) * kChannels * MAT + (size_t)src * MAT;
+          const double2* ps = st->P + (size_t)(n & 31) * kChannels * MAT + (size_t)src * MAT;
           double2 a[BB / 32], b[BB / 32];
 #pragma unroll
           for (int q = 0; q < BB / 32; ++q) {   // element q * 32 + lane of the tile
@@ -593,14 +643,25 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
           flag_release(&sy->pflag[c0][rank], n);
         }
       };
-      serve();
+      serve([] {});
       team_sync();
-      while (!S.dec.stop) {
-        for (int s = 1; s <= 12; ++s) serve();
-        team_sync();
-        team_sync();
-        if (S.dec.accept && S.dec.dense)
-          for (int s = 13; s < 16; ++s) serve();
+      for (unsigned attempt = 1; !S.dec.stop; ++attempt) {
+        const double t = S.dec.nt, h = S.dec.nh;
+        const bool spec = S.dec.spec != 0;
+        for (int s = 1; s <= 12; ++s) serve([] {});
+        if (spec) {
+          serve([&] { if (rank == 0) post(attempt); });
+          serve([] {});
+          if (rank == 0) collect(attempt, t, h);
+          serve([] {});
+        } else {
+          team_sync();
+          if (rank == 0) {
+            post(attempt);
+            collect(attempt, t, h);
+          }
+          team_sync();
+        }
       }
       team_sync();
       return;
@@ -624,7 +685,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
       during();
       cluster_wait_acquire();
     }
-    double2* const pw = gp + (size_t)(seq & 15) * pstep;
+    double2* const pw = gp + (size_t)(seq & 31) * pstep;
     // ------------------------------------------------ phase 1
     {
       const int nt = warp % NTB, mg = (warp / NTB) % G::MG1, sl = warp / (NTB * G::MG1);
@@ -716,7 +777,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
               const size_t off = (size_t)c * MAT + ((size_t)(bi * KS + bj * KB + kl) * MT + mt) * 128 + 32 * q + l;
               pw[off] = v;
               // a one-CTA team publishes P for the team that inserts it
-              if (NB == 1 && teams > 1) st->P[(size_t)(seq & 15) * VEC + off] = v;
+              if (NB == 1 && teams > 1) st->P[(size_t)(seq & 31) * VEC + off] = v;
             }
             if (ql) {
               const int r = el_r(it), col = el_c(it);
@@ -790,7 +851,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
         // the epilogue's operands, in flight during the products (B = 32 loads them after: registers)
         const int s = c_src[c];
         const bool remote = !SM::COMM && s >= 0 && (s < c0 || s >= c1);
-        const double2* ps = (remote ? st->P + (size_t)(seq & 15) * VEC : pw) + (size_t)(s >= 0 ? s : 0) * MAT;
+        const double2* ps = (remote ? st->P + (size_t)(seq & 31) * VEC : pw) + (size_t)(s >= 0 ? s : 0) * MAT;
         const double2* fx = c == 0 ? st->fixed0 : c == 6 ? st->fixed6 : nullptr;
         double2 ev[EPT], iv[EPT];   // Y's other half, the insertion P_s + P_s^dag
         auto operands = [&](int it) {
@@ -975,9 +1036,8 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
   rhs(k0slot, S.jac[0], S.src[0], [] {});
 
   const double atol = st->atol, rtol = st->rtol;
-  const double N = packed ? 10.0 * half * half + 1.0 : (double)kChannels * st->d * st->d + 1.0;
   const unsigned long long t_start = global_ns();
-  if (rank == 0 && warp == 0) first_decision<NR>(S, st, ctl_in);
+  if (rank == 0 && warp == 0) first_decision<NR>(S, st, ctl_in, points, npoints);
   team_sync();
 
   unsigned attempt = 0;
@@ -985,6 +1045,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
   while (!stop) {
     ++attempt;
     const double t = S.dec.nt, h = S.dec.nh;
+    const bool spec = S.dec.spec != 0;
     block_sync();
     stage_times(S, t, h);
     block_sync();
@@ -1064,39 +1125,22 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
       else if constexpr (NR == 1) s_gat[tid] = x;
       else dsmem_store_f64(s_gat + rank * SM::NREC + tid, 0, x);
     }
-    team_sync();
-    if (rank == 0 && warp == 0) {
-      // lane v: entry v of the team's record, summed over its CTAs
-      double tot = 0.0;
-      const int own = !LONE ? lane : lane >= 14 ? lane - 12 : lane == c0 ? 0 : lane == 7 + c0 ? 1 : -1;
-      if (lane < kRec && own >= 0)
-        for (int g = 0; g < NR; ++g)
-          tot += SM::GLOBAL_REC ? __ldcg(&sy->crec[team][g][own]) : s_gat[SM::NREC * g + own];
-      const long long next = C.next_point;
-      double pt = next + lane < npoints ? points[next + lane] : INFINITY;
-      if (teams > 1) {
-        const int par = attempt & 1;
-        if (lane < kRec) sy->rec[team][par][lane] = tot;
-        __syncwarp();
-        if (lane == 0) {
-          __threadfence();
-          flag_release(&sy->rflag[team], attempt);
-        }
-        if (lane < teams) flag_wait(&sy->rflag[lane], attempt, &S.wait_flag);
-        __syncwarp();
-        tot = 0.0;
-        if (lane < kRec)
-          for (int g = 0; g < teams; ++g) tot += __ldcg(&sy->rec[g][par][lane]);
-        if (lane == 18 && S.wait_flag) tot = 1.0;
+    bool dense = SM::COMM && spec;
+    if constexpr (SM::COMM) {
+      if (!spec) {
+        team_sync();
+        team_sync();
       }
-      if (lane < kRec) S.tot[lane] = tot;
-      __syncwarp();
-      decide<NR>(S, st, ctl_in, points, npoints, pt, N, t, h);
+    } else {
+      team_sync();
+      if (rank == 0 && warp == 0) {
+        post(attempt);
+        collect(attempt, t, h);
+      }
+      team_sync();
+      dense = S.dec.accept && S.dec.dense;
     }
-    team_sync();
-    stop = S.dec.stop != 0;
-    if (S.dec.accept) {
-      if (S.dec.dense) {
+    if (dense) {
         // dense stages 13..15
         partial_sum(c_dop_a + 16 * 13, 12, h, std::integral_constant<int, 12>());
         for (int s = 13; s < 16; ++s) {
@@ -1116,6 +1160,10 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
             if (s < 15) partial_sum(c_dop_a + 16 * (s + 1), s, h, std::integral_constant<int, 14>());
           });
         }
+    }
+    stop = S.dec.stop != 0;
+    if (S.dec.accept) {
+      if (dense) {
         // order-7 interpolation at the nodes in (t, t_new]
         const double tn = S.dec.tn;
         const long long first = S.dec.first, last = S.dec.last;
@@ -1449,7 +1497,7 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
   const double atol = st->atol, rtol = st->rtol;
   const double N = packed ? 10.0 * half * half + 1.0 : (double)kChannels * st->d * st->d + 1.0;
   const unsigned long long t_start = global_ns();
-  if (rank == 0 && warp == 0) first_decision<NR>(S, st, ctl_in);
+  if (rank == 0 && warp == 0) first_decision<NR>(S, st, ctl_in, points, npoints);
   team_sync();
 
   bool stop = S.dec.stop != 0;
