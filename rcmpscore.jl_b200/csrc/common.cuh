@@ -228,6 +228,14 @@ RCMPS_DEVICE_INLINE double dsmem_load(const double* p, uint32_t rank) {
   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(remote) : "memory");
   return v;
 }
+// Read a complex value from the shared memory of CTA `rank`.
+RCMPS_DEVICE_INLINE double2 dsmem_load_z(const double2* p, uint32_t rank) {
+  uint32_t local = smem_u32(p), remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  double2 v;
+  asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(remote) : "memory");
+  return v;
+}
 // Write a double into the shared memory of CTA `rank` of this cluster (visible there after the next
 // cluster barrier).
 RCMPS_DEVICE_INLINE void dsmem_store_f64(double* p, uint32_t rank, double v) {

@@ -199,6 +199,173 @@ lindblad_kernel(const LindbladTask* __restrict__ tasks, const ArnoldiProblem* __
   if (tid == 0 && *flag && T.flag) atomicExch(T.flag, 1);
 }
 
+// The same action for few problems, on square tiles: a cluster of NB^2 CTAs per problem, CTA (i, j)
+// with tile (i, j) of
+//   out = [A1_i | X_i] [X_j; A1h_j] + P_i A2h_j,  P_ij = A2_i X_j.
+// Bound by latency (a GMRES step waits for one action), so it takes NB times the SMs of the row-block
+// form, splits K over the warps, reads every fragment straight from L2 and exchanges the P tiles
+// through distributed shared memory: one problem at D = 64 24.5 -> 9 us.
+template <int DP>
+struct LTile {
+  static constexpr int B = DP <= 64 ? 16 : 32, NB = DP / B, NR = NB * NB;
+  static constexpr int KS = DP / 8, KB = B / 8, MT = B / 16, NTB = B / 8;
+  static constexpr int NW = DP == 48 ? 12 : 8, NT = 32 * NW, S = NW / NTB, K = (KS + S - 1) / S;
+  static constexpr int OWN = 256, EPT = B * B / OWN;
+  static constexpr int RED = S * 2 * MT * NTB * 128, PT = B * B;
+  static constexpr size_t SMEM = (size_t)(RED + PT) * 16;
+};
+
+template <int DP>
+__global__ void __launch_bounds__(LTile<DP>::NT)
+lindblad_tile_kernel(const LindbladTask* __restrict__ tasks, const ArnoldiProblem* __restrict__ probs, int j) {
+  using L = LTile<DP>;
+  constexpr int B = L::B, NB = L::NB, KS = L::KS, KB = L::KB, MT = L::MT, NTB = L::NTB, S = L::S;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  double2* red = reinterpret_cast<double2*>(smem_raw);   // [S][2 MT NTB][128] partial tiles: U, then P
+  double2* pt = red + L::RED;                            // [KB][MT][4][32] the P tile, A-fragment order
+  __shared__ double2 tr_gat[16];                         // every CTA's part of the trace
+  __shared__ double2 tr_red[L::NW];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int task = blockIdx.x / L::NR, rank = (int)cluster_rank();
+  const LindbladTask T = tasks ? tasks[task] : arnoldi_task(probs[task], j);
+  if (!T.X) return;   // inactive slot: the whole cluster
+  const int bi = rank / NB, bj = rank % NB, r0 = bi * B, c0 = bj * B;
+  const int nt = warp % NTB, sl = warp / NTB;
+  cluster_arrive_release();   // every CTA runs before the others write into it (awaited below)
+  auto frag_b = [&](const double2* M, int ks, BFrag& b) {   // rows 8 ks.., columns c0 + 8 nt..
+    const double2* p = M + (size_t)(8 * ks + t) * DP + c0 + 8 * nt + g;
+    const double2 v0 = p[0], v1 = p[4 * DP];
+    b.r[0] = v0.x; b.r[1] = v1.x;
+    b.i[0] = v0.y; b.i[1] = v1.y;
+    b.s[0] = v0.x + v0.y; b.s[1] = v1.x + v1.y;
+  };
+  auto to_a = [&](double2 v0, double2 v1, double2 v2, double2 v3, AFrag& a) {
+    a.r[0] = v0.x; a.r[1] = v1.x; a.r[2] = v2.x; a.r[3] = v3.x;
+    a.i[0] = v0.y; a.i[1] = v1.y; a.i[2] = v2.y; a.i[3] = v3.y;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a.s[q] = a.r[q] + a.i[q];
+  };
+  auto frag_a = [&](const double2* M, int m, int ks, AFrag& a) {   // rows r0 + 16 m.., columns 8 ks..
+    const double2* p = M + (size_t)(r0 + 16 * m + g) * DP + 8 * ks + t;
+    to_a(p[0], p[8 * DP], p[4], p[8 * DP + 4], a);
+  };
+  ZFrag u[MT], pp[MT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    u[m].zero();
+    pp[m].zero();
+  }
+#pragma unroll (DP <= 64 ? L::K : 2)
+  for (int q = 0; q < L::K; ++q) {
+    const int ks = sl + q * S;
+    if (ks >= KS) break;
+    BFrag bx, bh;
+    frag_b(T.X, ks, bx);
+    frag_b(T.A1h, ks, bh);
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      AFrag a1, a2, ax;
+      frag_a(T.A1, m, ks, a1);
+      frag_a(T.A2, m, ks, a2);
+      frag_a(T.X, m, ks, ax);
+      zmma(u[m], a1, bx);
+      zmma(pp[m], a2, bx);
+      zmma(u[m], ax, bh);
+    }
+  }
+  // the CTA's part of tr(trw X) = sum trw_ab X_ba over its tile
+  if (T.trw) {
+    double2 v = make_double2(0, 0);
+    for (int e = tid; e < B * B; e += L::NT) {
+      const int a = r0 + e / B, b = c0 + e % B;
+      v = zadd(v, zmul(T.trw[(size_t)a * DP + b], T.X[(size_t)b * DP + a]));
+    }
+    v.x = warp_sum(v.x);
+    v.y = warp_sum(v.y);
+    if (lane == 0) tr_red[warp] = v;
+  }
+  auto deposit = [&](const ZFrag* acc, int part) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      double2* p = red + ((size_t)(sl * 2 + part) * MT * NTB + m * NTB + nt) * 128 + lane;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[32 * i] = acc[m].value(i);
+    }
+  };
+  // entry (r, c) of a product summed over its slices
+  auto total = [&](int part, int r, int c) {
+    const double2* p = red + ((size_t)part * MT * NTB + (r / 16) * NTB + c / 8) * 128 +
+                       (2 * ((r >> 3) & 1) + (c & 1)) * 32 + 4 * (r & 7) + ((c & 7) >> 1);
+    double2 v = p[0];
+#pragma unroll
+    for (int s = 1; s < S; ++s) v = zadd(v, p[(size_t)s * 2 * MT * NTB * 128]);
+    return v;
+  };
+  deposit(u, 0);
+  deposit(pp, 1);
+  __syncthreads();
+  cluster_wait_acquire();
+  double2 uv[L::EPT];
+  if (tid < L::OWN) {
+#pragma unroll
+    for (int it = 0; it < L::EPT; ++it) {
+      const int e = it * L::OWN + tid, l = e & 31, q = (e >> 5) & 3;
+      const int kl = e / (128 * MT), mt = (e >> 7) % MT;
+      pt[e] = total(1, 16 * mt + (l >> 2) + 8 * (q & 1), 8 * kl + (l & 3) + 4 * (q >> 1));
+      uv[it] = total(0, 16 * (e / (128 * NTB)) + 8 * ((e >> 6) & 1) + ((e >> 2) & 7),
+                     8 * ((e / 128) % NTB) + 2 * (e & 3) + ((e >> 5) & 1));
+    }
+  }
+  if (T.trw && tid < L::NR) {
+    double2 v = make_double2(0, 0);
+    for (int w = 0; w < L::NW; ++w) v = zadd(v, tr_red[w]);
+    dsmem_store_f64(&tr_gat[rank].x, (uint32_t)tid, v.x);
+    dsmem_store_f64(&tr_gat[rank].y, (uint32_t)tid, v.y);
+  }
+  cluster_sync();   // every P tile and every part of the trace is in place
+  ZFrag acc[MT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) acc[m].zero();
+#pragma unroll (DP <= 64 ? L::K : 2)
+  for (int q = 0; q < L::K; ++q) {
+    const int ks = sl + q * S;
+    if (ks >= KS) break;
+    BFrag b;
+    frag_b(T.A2h, ks, b);
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      double2 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        v[i] = dsmem_load_z(pt + ((ks % KB) * MT + m) * 128 + 32 * i + lane, (uint32_t)(bi * NB + ks / KB));
+      AFrag a;
+      to_a(v[0], v[1], v[2], v[3], a);
+      zmma(acc[m], a, b);
+    }
+  }
+  cluster_arrive_release();   // done with the other CTAs' P tiles (awaited before the exit)
+  deposit(acc, 0);
+  __syncthreads();
+  if (tid < L::OWN) {
+    double2 tr = make_double2(0, 0);
+    if (T.trw)
+      for (int r = 0; r < L::NR; ++r) tr = zadd(tr, tr_gat[r]);
+#pragma unroll
+    for (int it = 0; it < L::EPT; ++it) {
+      const int e = it * L::OWN + tid;
+      const int r = 16 * (e / (128 * NTB)) + 8 * ((e >> 6) & 1) + ((e >> 2) & 7);
+      const int c = 8 * ((e / 128) % NTB) + 2 * (e & 3) + ((e >> 5) & 1);
+      double2 v = zadd(total(0, r, c), uv[it]);
+      if (T.trw) {
+        v = make_double2(-v.x, -v.y);
+        if (r0 + r == c0 + c && r0 + r < T.d) v = zadd(v, tr);
+      }
+      T.out[(size_t)(r0 + r) * DP + c0 + c] = v;
+    }
+  }
+  cluster_wait_acquire();
+}
+
 // ======================================================================= Gram-Schmidt passes
 // One CTA per (chunk of CH rows, problem). Problem data: ArnoldiProblem.
 constexpr int CH = 512;
@@ -1139,10 +1306,40 @@ __global__ void residual_reduce(ArnoldiProblem* __restrict__ probs, int nprob, c
 }
 
 // ======================================================================= launchers
+// The tile form takes up to this many CTAs: one or two problems at D = 64 and 128, eight at D = 32. Its
+// clusters want an SM per CTA in one GPC, which more problems beside a trajectory would not find.
+constexpr int kTileCtas = 32;
+
+template <int DP>
+static cudaError_t launch_l_tile(const LindbladTask* tasks, const ArnoldiProblem* probs, int j, int ntasks,
+                                 cudaStream_t s) {
+  using L = LTile<DP>;
+  auto k = lindblad_tile_kernel<DP>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ntasks * L::NR, 1, 1);
+  cfg.blockDim = dim3(L::NT, 1, 1);
+  cfg.dynamicSmemBytes = L::SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = L::NR;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  note_launch();
+  return cudaLaunchKernelEx(&cfg, k, tasks, probs, j);
+}
+
 template <int DP>
 static cudaError_t launch_l(const LindbladTask* tasks, const ArnoldiProblem* probs, int j, int ntasks, int mode,
                             cudaStream_t s) {
   using LG = LGeo<DP>;
+  if constexpr (DP >= 32)
+    if (mode == 0 && ntasks > 0 && ntasks * LTile<DP>::NR <= kTileCtas) return launch_l_tile<DP>(tasks, probs, j, ntasks, s);
   auto k = lindblad_kernel<DP>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LG::SMEM);
   if (e != cudaSuccess) return e;
