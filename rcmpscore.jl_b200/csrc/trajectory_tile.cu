@@ -10,8 +10,7 @@
 // only, and the mirrored entry is written, never computed: X_c is Hermitian to the last bit.
 //
 // Layout. A matrix is cut into NB x NB tiles of B x B (B = 16 up to DP = 64, 32 above). A team of
-// NB^2 CTAs, one cluster, holds one tile each of the channels [c0, c1) of a state; a state has 1, 2,
-// 4 or 7 teams. CTA (i, j):
+// NB^2 CTAs, one cluster, holds one tile each of one channel of a state, or of all seven. CTA (i, j):
 //   phase 1: Y_c(i, j) and P_c(i, j): A = [Qc; Rc] rows of block i (shared memory, constant), B = the
 //            columns j of X_c;
 //   phase 2: T = (P_c Rc^dag)(i, j) when the CTA owns that tile of the channel (i = j, or one of
@@ -28,7 +27,8 @@
 // tile and right-hand side, and only towards the channels that follow in the chains 0 -> 1 -> 2 and
 // 6 -> 5 -> 4 -> 3, so a team runs ahead of its followers and nobody waits inside an attempt for a
 // team behind it; the teams meet once per attempt at the error norm. Teams of one state wait for one
-// another, so such a launch is cooperative. A batch that fills the GPU takes one team per state.
+// another, so such a launch is cooperative. A batch takes one team per state (wide_kernel up to
+// DP = 64) when that is faster than a few states at a time (use_teams).
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
@@ -46,9 +46,6 @@ constexpr int kChannels = 7;
 __constant__ int c_src[kChannels] = {-1, 0, 1, 4, 5, 6, -1};
 __constant__ double c_coef[kChannels] = {0.0, 2.0, 3.0, 1.0, 2.0, 3.0, 0.0};
 __constant__ int c_feeds[kChannels] = {1, 2, -1, -1, 3, 4, 5};
-// channels of team t when a state has 1, 2, 4 or 7 teams (first channel, count)
-__constant__ int c_first[4][7] = {{0}, {0, 3}, {0, 2, 3, 5}, {0, 1, 2, 3, 4, 5, 6}};
-__constant__ int c_count[4][7] = {{7}, {3, 4}, {2, 1, 2, 2}, {1, 1, 1, 1, 1, 1, 1}};
 
 constexpr int kMaxTiles = 16;
 // A record: 0..6 and 7..13 the two error sums by channel; 14..17 the scalar channel's part of the
@@ -63,7 +60,7 @@ struct Sync {
   unsigned pflag[kChannels][kMaxTiles];      // right-hand sides whose P tile is complete
   unsigned rflag[8];                         // attempts whose record is complete, by team
   double rec[kChannels][2][kRec];            // a team's sums, by the attempt's parity
-  double crec[4][kMaxTiles][kRec];           // the CTAs' records of a team whose rank 0 has no room for them
+  double crec[kMaxTiles][kRec];              // the CTAs' records of a team whose rank 0 has no room for them
 };
 
 template <int DP>
@@ -464,7 +461,7 @@ __device__ __forceinline__ double2 dense_value(const double2* cf, double2 yo, do
 template <int DP, bool LONE>
 __global__ void __launch_bounds__(Smem<DP, LONE>::THREADS, 1)
 tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ points, int npoints, TrajControls ctl_in,
-            Sync* __restrict__ sync, int teams, int level) {
+            Sync* __restrict__ sync) {
   using G = TG<DP>;
   using SM = Smem<DP, LONE>;
   constexpr int B = G::B, NB = G::NB, NR = G::NR, KS = G::KS, KB = G::KB, MT = G::MT, NTB = G::NTB;
@@ -473,12 +470,13 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = NR == 1 ? 0 : (int)cluster_rank();
+  constexpr int teams = LONE ? kChannels : 1;
   const int cid = blockIdx.x / NR;
   const int sidx = cid / teams, team = cid % teams;
   const TrajState* st = states + sidx;
   if (!st->herm || st->z2 < 0) return;    // the state's whole grid of CTAs leaves here
   Sync* sy = sync + sidx;
-  const int c0 = c_first[level][team], c1 = c0 + c_count[level][team];
+  const int c0 = LONE ? team : 0, c1 = LONE ? team + 1 : kChannels;   // the team's channels
   const int bi = rank / NB, bj = rank % NB;   // tile (i, j)
   const bool owner_thread = tid < G::OWN;
 
@@ -581,7 +579,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
     team_tot = 0.0;
     if (lane < kRec && own >= 0)
       for (int g = 0; g < NR; ++g)
-        team_tot += SM::GLOBAL_REC ? __ldcg(&sy->crec[team][g][own]) : s_gat[SM::NREC * g + own];
+        team_tot += SM::GLOBAL_REC ? __ldcg(&sy->crec[g][own]) : s_gat[SM::NREC * g + own];
     if (teams > 1) {
       if (lane < kRec) sy->rec[team][attempt & 1][lane] = team_tot;
       __syncwarp();
@@ -1121,7 +1119,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
       const int v = !LONE ? tid : tid < 2 ? 7 * tid + c0 : tid + 12;
       const double x = record_entry(S, v, G::NW, c0, c1, h, ctl_in.max_ns && global_ns() - t_start >= ctl_in.max_ns,
                                     [&](int q, int c, int i) { return s_we[(q * SM::NC + (LONE ? 0 : c)) * G::NW + i]; });
-      if constexpr (SM::GLOBAL_REC) sy->crec[team][rank][tid] = x;
+      if constexpr (SM::GLOBAL_REC) sy->crec[rank][tid] = x;
       else if constexpr (NR == 1) s_gat[tid] = x;
       else dsmem_store_f64(s_gat + rank * SM::NREC + tid, 0, x);
     }
@@ -1694,50 +1692,69 @@ static int resident_clusters(K kern, int threads, size_t smem) {
   return n;
 }
 
+// States whose seven teams are resident at once, and those of the one-team kernel.
 template <int DP>
-static int teams_for(int nstates) {
-  using G = TG<DP>;
+static int lone_states() {
   static_assert(Smem<DP, true>::bytes() <= 232448, "shared memory per CTA");
-  if ((long long)nstates * 7 <= resident_clusters<DP>(tile_kernel<DP, true>, Smem<DP, true>::THREADS, Smem<DP, true>::bytes())) return 7;
-  if constexpr (G::B == 16) {
-    return resident_clusters<DP>(wide_kernel<DP>, Wide<DP>::NT, Wide<DP>::BYTES) >= 1 ? 1 : 0;
+  return resident_clusters<DP>(tile_kernel<DP, true>, Smem<DP, true>::THREADS, Smem<DP, true>::bytes()) / kChannels;
+}
+template <int DP>
+static int batch_states() {
+  if constexpr (TG<DP>::B == 16) {
+    return resident_clusters<DP>(wide_kernel<DP>, Wide<DP>::NT, Wide<DP>::BYTES);
   } else {
     static_assert(Smem<DP, false>::bytes() <= 232448, "shared memory per CTA");
-    const int n = resident_clusters<DP>(tile_kernel<DP, false>, G::NT, Smem<DP, false>::bytes());
-    for (int t : {4, 2})
-      if ((long long)nstates * t <= n) return t;
-    return n >= 1 ? 1 : 0;
+    return resident_clusters<DP>(tile_kernel<DP, false>, TG<DP>::NT, Smem<DP, false>::bytes());
   }
+}
+
+// Seven teams per state, a few states per launch one launch after another, or one team per state, as
+// many states at once as fit: the former while its rounds number at most 4 (DP <= 64) or 6 times the
+// latter's. Measured per right-hand side, one round of either: D = 16 2.8 against 14 us, D = 32 4.5
+// against 25, D = 48 5.3 against 21, D = 64 5.6 against 24, D = 96 20 against 130, D = 128 26 against 190.
+template <int DP>
+static int teams_for(int nstates) {
+  const int lone = lone_states<DP>(), batch = batch_states<DP>();
+  const long long rounds = lone ? (nstates + lone - 1) / lone : 0, waves = batch ? (nstates + batch - 1) / batch : 0;
+  if (lone && (!batch || rounds <= (TG<DP>::B == 16 ? 4 : 6) * waves)) return kChannels;
+  return batch ? 1 : 0;
+}
+
+template <int DP>
+static int ctas_for(int nstates) {
+  const int teams = teams_for<DP>(nstates);
+  return TG<DP>::NR * teams * std::min(nstates, teams == kChannels ? lone_states<DP>() : batch_states<DP>());
 }
 
 template <int DP>
 static cudaError_t launch(const TrajState* d_states, int nstates, const double* d_points, int npoints,
                           const TrajControls& ctl, void* sync, int teams, cudaStream_t stream) {
   using G = TG<DP>;
-  const int level = teams == 7 ? 3 : teams == 4 ? 2 : teams == 2 ? 1 : 0;
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg;
   cudaError_t e;
-  if (teams > 1) {
+  Sync* sy = static_cast<Sync*>(sync);
+  if (teams == kChannels) {
     e = cudaMemsetAsync(sync, 0, (size_t)nstates * sizeof(Sync), stream);
-    if (e != cudaSuccess) return e;
+    const int lone = lone_states<DP>();
+    for (int s = 0; e == cudaSuccess && s < nstates; s += lone) {
+      note_launch();
+      e = configure<DP>(tile_kernel<DP, true>, std::min(lone, nstates - s) * kChannels, Smem<DP, true>::THREADS,
+                        Smem<DP, true>::bytes(), true, stream, attr, cfg);
+      if (e == cudaSuccess)
+        e = cudaLaunchKernelEx(&cfg, tile_kernel<DP, true>, d_states + s, d_points, npoints, ctl, sy + s);
+    }
+    return e;
   }
   note_launch();
-  if (teams == 7) {
-    e = configure<DP>(tile_kernel<DP, true>, nstates * teams, Smem<DP, true>::THREADS, Smem<DP, true>::bytes(), true, stream,
-                      attr, cfg);
-    if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, tile_kernel<DP, true>, d_states, d_points, npoints, ctl, (Sync*)sync, teams, level);
-  }
   if constexpr (G::B == 16) {
     e = configure<DP>(wide_kernel<DP>, nstates, Wide<DP>::NT, Wide<DP>::BYTES, false, stream, attr, cfg);
     if (e != cudaSuccess) return e;
     return cudaLaunchKernelEx(&cfg, wide_kernel<DP>, d_states, d_points, npoints, ctl);
   } else {
-    e = configure<DP>(tile_kernel<DP, false>, nstates * teams, G::NT, Smem<DP, false>::bytes(), teams > 1, stream, attr,
-                      cfg);
+    e = configure<DP>(tile_kernel<DP, false>, nstates, G::NT, Smem<DP, false>::bytes(), false, stream, attr, cfg);
     if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, tile_kernel<DP, false>, d_states, d_points, npoints, ctl, (Sync*)sync, teams, level);
+    return cudaLaunchKernelEx(&cfg, tile_kernel<DP, false>, d_states, d_points, npoints, ctl, sy);
   }
 }
 
@@ -1763,8 +1780,15 @@ int tile_trajectory_teams(int dp, int nstates) {
 }
 
 int tile_trajectory_ctas(int dp, int nstates) {
-  const int teams = tile_trajectory_teams(dp, nstates), nb = dp <= 64 ? dp / 16 : dp / 32;
-  return nstates * teams * nb * nb;
+  switch (dp) {
+    case 16: return tile::ctas_for<16>(nstates);
+    case 32: return tile::ctas_for<32>(nstates);
+    case 48: return tile::ctas_for<48>(nstates);
+    case 64: return tile::ctas_for<64>(nstates);
+    case 96: return tile::ctas_for<96>(nstates);
+    case 128: return tile::ctas_for<128>(nstates);
+    default: return 0;
+  }
 }
 
 cudaError_t tile_trajectory_launch(int dp, const TrajState* d_states, int nstates, const double* d_points, int npoints,

@@ -51,7 +51,7 @@ def test_quartic_against_the_oracle(gpu_context, d, z2):
 def test_large_tiles_against_the_row_blocks(gpu_context, d, z2):
     state = _state(d, z2, d)
     (e0, c0, v0, a0, r0), = _batch([state], groups=1)
-    for n in (1, 4, 9):     # one team per channel, several channels per team, one team
+    for n in (1, 4, 20):    # a lone state, a few launches of one team per channel, one team per state
         for e, c, v, a, r in _batch([state] * n):
             assert (a, r) == (a0, r0)
             assert abs(e - e0) <= 1e-12 * abs(e0)
@@ -59,7 +59,7 @@ def test_large_tiles_against_the_row_blocks(gpu_context, d, z2):
             assert np.linalg.norm(v - v0) <= 1e-11 * np.linalg.norm(v0)
 
 
-@pytest.mark.parametrize("d,many", [(9, 24), (16, 24), (24, 40), (32, 40), (40, 5), (48, 20), (50, 4), (64, 12)])
+@pytest.mark.parametrize("d,many", [(9, 100), (16, 24), (24, 40), (32, 40), (40, 5), (48, 20), (50, 4), (64, 12)])
 def test_batch_and_lone_state_give_the_same_bits(gpu_context, d, many):
     states = [_state(d, i % 2 == 1 and d % 2 == 0, 10 * d + i) for i in range(3)]
     batch = _batch([states[i % 3] for i in range(many)])
