@@ -1439,43 +1439,50 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
     if (bi != bj || r != col) z[zoff<DP>(bj, bi, col, r)] = zconj(v);
   };
 
-  // partial sums of the next stage vector and of the error estimates, in slots 18 and 19 (tile_kernel)
-  auto partial_sum = [&](const double* w, int n, double h, auto max) {
+  // Stage sums and error estimates as in tile_kernel: with one column tile per warp all but the last
+  // term is summed during the right-hand side before (slots 18 and 19); with two, where two CTAs share an
+  // SM and the stage vectors' L2 traffic sets the pace, when it is used.
+  constexpr bool EARLY = NPT == 1;
+  auto entry_sum = [&](const double* w, int n, double h, auto max, int e) -> double2 {
     constexpr int MAX = decltype(max)::value;
-    if (!own) return;
+    double2 kv[MAX];
 #pragma unroll
-    for (int it = 0; it < NPT; ++it)
+    for (int j = 0; j < MAX; ++j) kv[j] = j < n && w[j] != 0.0 ? kvec(kslot(j))[e] : make_double2(0.0, 0.0);
+    double2 v = kvec(yslot)[e];
+#pragma unroll
+    for (int j = 0; j < MAX; ++j) v = zaxpy(j < n ? h * w[j] : 0.0, kv[j], v);
+    return v;
+  };
+  auto entry_errors = [&](int e, double2& e5, double2& e3) {
+    double2 kv[12];
+#pragma unroll
+    for (int j = 0; j < 12; ++j) kv[j] = kvec(kslot(j))[e];
+    e5 = e3 = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int j = 0; j < 12; ++j) {
+      e5 = zaxpy(c_dop_e5[j], kv[j], e5);
+      e3 = zaxpy(c_dop_e3[j], kv[j], e3);
+    }
+  };
+  auto partial_sum = [&](const double* w, int n, double h, auto max) {
+    if constexpr (EARLY) {
+      if (!own) return;
 #pragma unroll 2
-      for (int i = 0; i < 4; ++i) {
-        const int e = el_e(nt0 + it, i);
-        double2 kv[MAX];
-#pragma unroll
-        for (int j = 0; j < MAX; ++j) kv[j] = j < n && w[j] != 0.0 ? kvec(kslot(j))[e] : make_double2(0.0, 0.0);
-        double2 v = kvec(yslot)[e];
-#pragma unroll
-        for (int j = 0; j < MAX; ++j) v = zaxpy(j < n ? h * w[j] : 0.0, kv[j], v);
-        kvec(18)[e] = v;
-      }
+      for (int i = 0; i < 4; ++i)
+        if (active(el_r(i), el_c(nt0, i))) kvec(18)[el_e(nt0, i)] = entry_sum(w, n, h, max, el_e(nt0, i));
+    }
   };
   auto partial_errors = [&]() {
-    if (!own) return;
-#pragma unroll
-    for (int it = 0; it < NPT; ++it)
+    if constexpr (EARLY) {
+      if (!own) return;
 #pragma unroll 1
       for (int i = 0; i < 4; ++i) {
-        const int e = el_e(nt0 + it, i);
-        double2 kv[12];
-#pragma unroll
-        for (int j = 0; j < 12; ++j) kv[j] = kvec(kslot(j))[e];
-        double2 e5 = make_double2(0.0, 0.0), e3 = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int j = 0; j < 12; ++j) {
-          e5 = zaxpy(c_dop_e5[j], kv[j], e5);
-          e3 = zaxpy(c_dop_e3[j], kv[j], e3);
-        }
-        kvec(18)[e] = e5;
-        kvec(19)[e] = e3;
+        double2 e5, e3;
+        entry_errors(el_e(nt0, i), e5, e3);
+        kvec(18)[el_e(nt0, i)] = e5;
+        kvec(19)[el_e(nt0, i)] = e3;
       }
+    }
   };
 
   // ---------------------------------------------------------------- start: y = 0, k0 = f(-a, 0)
@@ -1509,12 +1516,15 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
       if (own) {
 #pragma unroll
         for (int it = 0; it < NPT; ++it)
-#pragma unroll
+#pragma unroll (EARLY ? 4 : 2)
           for (int i = 0; i < 4; ++i) {
             const int nt = nt0 + it, r = el_r(i), col = el_c(nt, i), e = el_e(nt, i);
             double part = 0.0;
             if (active(r, col)) {
-              const double2 v = zaxpy(h * w[s - 1], kvec(kslot(s - 1))[e], kvec(s == 1 ? yslot : 18)[e]);
+              double2 base;
+              if constexpr (EARLY) base = kvec(s == 1 ? yslot : 18)[e];
+              else base = entry_sum(w, s - 1, h, std::integral_constant<int, 11>(), e);
+              const double2 v = zaxpy(h * w[s - 1], kvec(kslot(s - 1))[e], base);
               put_z(r, col, v);
               if (s == 12) kvec(pslot)[e] = v;
               if (c == 2) {
@@ -1544,7 +1554,15 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
           const double wt = active(r, col) ? norm_weight(packed, half, c, bi * B + r, bj * B + col) : 0.0;
           if (wt != 0.0) {
             const double2 k12 = kvec(kslot(12))[e];
-            const double2 e5 = zaxpy(c_dop_e5[12], k12, kvec(18)[e]), e3 = zaxpy(c_dop_e3[12], k12, kvec(19)[e]);
+            double2 e5, e3;
+            if constexpr (EARLY) {
+              e5 = kvec(18)[e];
+              e3 = kvec(19)[e];
+            } else {
+              entry_errors(e, e5, e3);
+            }
+            e5 = zaxpy(c_dop_e5[12], k12, e5);
+            e3 = zaxpy(c_dop_e3[12], k12, e3);
             const double2 yo = kvec(yslot)[e], yn = kvec(pslot)[e];
             const double scale = atol + rtol * fmax(hypot(yo.x, yo.y), hypot(yn.x, yn.y));
             s5 += wt * (zabs2(e5) / (scale * scale));
@@ -1585,11 +1603,14 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
           if (own) {
 #pragma unroll
             for (int it = 0; it < NPT; ++it)
-#pragma unroll
+#pragma unroll 1
               for (int i = 0; i < 4; ++i) {
                 const int nt = nt0 + it, r = el_r(i), col = el_c(nt, i), e = el_e(nt, i);
                 if (!active(r, col)) continue;
-                put_z(r, col, zaxpy(h * c_dop_a[16 * s + s - 1], kvec(kslot(s - 1))[e], kvec(18)[e]));
+                double2 base;
+                if constexpr (EARLY) base = kvec(18)[e];
+                else base = entry_sum(c_dop_a + 16 * s, s - 1, h, std::integral_constant<int, 14>(), e);
+                put_z(r, col, zaxpy(h * c_dop_a[16 * s + s - 1], kvec(kslot(s - 1))[e], base));
               }
           }
           rhs(s, S.jac[s], S.src[s], [&] {
