@@ -547,15 +547,58 @@ constexpr size_t kCgsMaxShared = 200 * 1024;
 
 __host__ __device__ inline int cgs_rows(int n, int g) { return ((n + g - 1) / g + 127) / 128 * 128; }
 inline size_t cgs_shared(int n, int g, int j) {
-  return ((size_t)cgs_rows(n, g) + kCgsThreads + (size_t)(g + 1) * (j + 1)) * sizeof(double2);
+  return ((size_t)cgs_rows(n, g) + kCgsThreads + (size_t)(g + 4) * (j + 1)) * sizeof(double2);
 }
 // CTAs per problem: 128 rows each, up to 16, and at most max_ctas for all problems where that leaves at
 // least one; fewer when the gathered projections would not fit; 0: this form does not fit.
 inline int cgs_cluster(int n, int j, int nprob, int max_ctas) {
-  int g = n >= 2048 ? 16 : n >= 1024 ? 8 : n >= 512 ? 4 : n >= 256 ? 2 : 1;
+  int g = n >= 2048 ? 16 : n >= 1024 ? 8 : n >= 512 ? 4 : 1;
   while (g > 1 && (long long)nprob * g > max_ctas && cgs_rows(n, g / 2) <= kCgsMaxRows) g /= 2;
   while (g > 1 && cgs_shared(n, g, j) > kCgsMaxShared) g /= 2;
   return cgs_rows(n, g) <= kCgsMaxRows && cgs_shared(n, g, j) <= kCgsMaxShared ? g : 0;
+}
+
+// The new column of a GMRES problem's Hessenberg matrix: the earlier rotations, the new one, the rotated
+// residual and the stop test (gmres_givens, by one thread), on the column hc and the rotations in shared
+// memory. In the Gram-Schmidt launch it costs 2 us; as a launch of its own, one thread reading column and
+// rotations from global memory took 7 us and a launch gap.
+__device__ void gmres_rotate(ArnoldiProblem& P, int j, const double2* hc, const double2* cs, const double2* sn,
+                             double beta) {
+  const int ld = P.kmax;
+  double2 a = hc[0];
+  for (int i = 0; i < j; ++i) {
+    const double c = cs[i].x;
+    const double2 s = sn[i], b = hc[i + 1];
+    P.H[(size_t)i * ld + j] = zadd(zscale(c, a), zmul(s, b));
+    a = zsub(zscale(c, b), zmul(zconj(s), a));
+  }
+  const double na = hypot(a.x, a.y), nb = fabs(beta);
+  double c;
+  double2 s;
+  if (na == 0.0) {
+    c = 0.0;
+    s = make_double2(1.0, 0.0);
+  } else {
+    const double r = hypot(na, nb);
+    c = na / r;
+    s = zscale(1.0 / r, zmul(make_double2(a.x / na, a.y / na), make_double2(beta, 0.0)));
+  }
+  P.cs[j] = make_double2(c, 0.0);
+  P.sn[j] = s;
+  P.H[(size_t)j * ld + j] = zadd(zscale(c, a), zmul(s, make_double2(beta, 0.0)));
+  P.H[(size_t)(j + 1) * ld + j] = make_double2(0, 0);
+  const double2 gj = P.g[j], gn = zscale(-1.0, zmul(zconj(s), gj));
+  P.g[j + 1] = gn;
+  P.g[j] = zscale(c, gj);
+  const double res = hypot(gn.x, gn.y);
+  P.gres = res;
+  P.iters += 1;
+  if (!isfinite(res)) {
+    P.nonfinite = 1;
+    P.active = 0;
+  } else if (res <= P.gtarget || P.exhausted || j + 1 >= P.target) {
+    P.active = 0;
+  }
 }
 
 __global__ void __launch_bounds__(kCgsThreads) cgs_fused(ArnoldiProblem* __restrict__ probs, int nprob, int j) {
@@ -569,6 +612,9 @@ __global__ void __launch_bounds__(kCgsThreads) cgs_fused(ArnoldiProblem* __restr
   double2* part = w + rows;                // [kCgsThreads]: the subtraction's partial sums
   double2* h = part + kCgsThreads;         // [m]: the summed projections
   double2* gat = h + m;                    // [G][m]: every CTA's projections
+  double2* hc = gat + (size_t)G * m;       // [m], GMRES, CTA 0: the column of H and the rotations so far
+  double2 *cs_sh = hc + m, *sn_sh = cs_sh + m;
+  const bool gmres = P.cs != nullptr;
   __shared__ double red[kCgsThreads / 32];
   __shared__ double nrm_sh[3][16];         // |w|^2 before, after each pass, of every CTA
   const int r0 = ch * rows, r1 = min(n, r0 + rows);
@@ -598,6 +644,11 @@ __global__ void __launch_bounds__(kCgsThreads) cgs_fused(ArnoldiProblem* __restr
     // before the first projection w = L(V_j): kept for the true residuals of the shifted solves
     if (P.LV && r0 + r < r1) P.LV[(size_t)j * P.ldv + r0 + r] = v;
   }
+  if (gmres && ch == 0)
+    for (int i = threadIdx.x; i < j; i += kCgsThreads) {
+      cs_sh[i] = P.cs[i];
+      sn_sh[i] = P.sn[i];
+    }
   cluster_sync();   // every CTA runs before the others write into it
   share_sum(s0, 0);
   double before = 0.0, after = 0.0;
@@ -656,7 +707,7 @@ __global__ void __launch_bounds__(kCgsThreads) cgs_fused(ArnoldiProblem* __restr
       double2 t = make_double2(0, 0);
       for (int g = 0; g < G; ++g) t = zadd(t, gat[(size_t)g * m + i]);
       h[i] = t;
-      if (ch == 0) P.H[(size_t)i * P.kmax + j] = zadd(P.H[(size_t)i * P.kmax + j], t);
+      if (ch == 0) P.H[(size_t)i * P.kmax + j] = hc[i] = zadd(P.H[(size_t)i * P.kmax + j], t);
     }
     __syncthreads();
     double nrm = 0.0;
@@ -705,6 +756,7 @@ __global__ void __launch_bounds__(kCgsThreads) cgs_fused(ArnoldiProblem* __restr
     P.k = j + 1;
     if (!isfinite(beta)) P.nonfinite = 1;
     if (exhausted) P.exhausted = 1;
+    if (gmres) gmres_rotate(P, j, hc, cs_sh, sn_sh, beta);
   }
 }
 
@@ -1338,8 +1390,8 @@ template <int DP>
 static cudaError_t launch_l(const LindbladTask* tasks, const ArnoldiProblem* probs, int j, int ntasks, int mode,
                             cudaStream_t s) {
   using LG = LGeo<DP>;
-  if constexpr (DP >= 32)
-    if (mode == 0 && ntasks > 0 && ntasks * LTile<DP>::NR <= kTileCtas) return launch_l_tile<DP>(tasks, probs, j, ntasks, s);
+  if (mode == 0 && ntasks > 0 && ntasks * LTile<DP>::NR <= kTileCtas)
+    return launch_l_tile<DP>(tasks, probs, j, ntasks, s);
   auto k = lindblad_kernel<DP>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LG::SMEM);
   if (e != cudaSuccess) return e;
@@ -1422,7 +1474,8 @@ cudaError_t cgs_fused_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, i
   return cudaLaunchKernelEx(&cfg, cgs_fused, d_probs, nprob, j);
 }
 
-cudaError_t gram_schmidt_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int sms, int spare, cudaStream_t s) {
+cudaError_t gram_schmidt_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int sms, int spare, cudaStream_t s,
+                                bool* rotated) {
   // Few problems: the step is latency-bound and one clustered launch wins. Its CTAs take an SM each and
   // a cluster one GPC, so beside a trajectory that leaves `spare` SMs it takes half of those: clusters
   // of 16 beside a lone D = 64 trajectory (112 SMs) found one GPC and ran one after another (kinetic
@@ -1431,8 +1484,9 @@ cudaError_t gram_schmidt_launch(ArnoldiProblem* d_probs, int nprob, int j, int n
   // clusters waiting at their barriers.
   const int few = (n + CH - 1) / CH < 8 ? (n + CH - 1) / CH : 8;
   const int limit = spare >= sms ? sms : spare / 2;
-  if ((long long)nprob * few <= 2ll * sms && cgs_cluster(n, j, nprob, limit))
-    return cgs_fused_launch(d_probs, nprob, j, n, limit, s);
+  const bool fused = (long long)nprob * few <= 2ll * sms && cgs_cluster(n, j, nprob, limit);
+  if (rotated) *rotated = fused;
+  if (fused) return cgs_fused_launch(d_probs, nprob, j, n, limit, s);
   return cgs_step_launch(d_probs, nprob, j, n, s);
 }
 

@@ -84,12 +84,14 @@ cudaError_t arnoldi_tasks_launch(const ArnoldiProblem* d_probs, int nprob, int j
                                 cudaStream_t s);
 cudaError_t arnoldi_start_launch(ArnoldiProblem* d_probs, int nprob, cudaStream_t s);
 cudaError_t cgs_step_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, cudaStream_t s);
-// The same Gram-Schmidt step in one launch (a cluster per problem, max_ctas for all of them where that
+// The same Gram-Schmidt step in one launch, with the Givens step of GMRES problems (a cluster per problem, max_ctas for all of them where that
 // leaves at least one; no partial or norm arrays).
 cudaError_t cgs_fused_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int max_ctas, cudaStream_t s);
 // The Gram-Schmidt step by whichever of the two forms suits the batch (sms: the device's SMs; spare:
-// those that work running beside this leaves free).
-cudaError_t gram_schmidt_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int sms, int spare, cudaStream_t s);
+// those that work running beside this leaves free). The one-launch form also does the Givens step of
+// GMRES problems (cs set); *rotated says whether it was taken.
+cudaError_t gram_schmidt_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int sms, int spare, cudaStream_t s,
+                                bool* rotated = nullptr);
 // W = L(V_j) (or L(Z_j)) of step j of every problem still extending, the task built in the kernel.
 cudaError_t lindblad_arnoldi_launch(int dp, const ArnoldiProblem* d_probs, int nprob, int j, cudaStream_t s);
 cudaError_t hessenberg_launch(ArnoldiProblem* d_probs, int nprob, const double* d_shifts, int nshift,

@@ -191,8 +191,7 @@ extern "C" int rcmps_finish_gradient_noalloc(rcmps_context* ctx, int d, const do
     for (int j = 0; j < m && !e; ++j) {
       e = arnoldi_tasks_launch(d_prob, 1, j, task, s);
       if (!e) e = lindblad_launch(dp, task, 1, 0, s);
-      if (!e) e = cgs_fused_launch(d_prob, 1, j, dp * dp, 16, s);
-      if (!e) e = gmres_givens_launch(d_prob, 1, j, s);
+      if (!e) e = cgs_fused_launch(d_prob, 1, j, dp * dp, 16, s);   // with the Givens step
     }
     if (!e) e = gmres_update_launch(d_prob, 1, dp * dp, m, s);
   }

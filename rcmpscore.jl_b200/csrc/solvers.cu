@@ -168,13 +168,34 @@ __global__ void gmres_update(ArnoldiProblem* __restrict__ probs, int nprob, int 
   if (P.converged || P.k == 0) return;
   extern __shared__ double2 y[];
   const int k = P.k, ld = P.kmax;
-  if (threadIdx.x == 0) {
-    for (int i = k - 1; i >= 0; --i) {
-      double2 s = P.g[i];
-      for (int q = i + 1; q < k; ++q) s = zsub(s, zmul(P.H[i * ld + q], y[q]));
-      const double2 d = P.H[i * ld + i];
-      const double den = zabs2(d);
-      y[i] = den > 0.0 ? zscale(1.0 / den, zmul(s, zconj(d))) : make_double2(0, 0);
+  // back substitution by one warp, a row of the triangle per lane and 32 columns at a time (one thread
+  // with its loads one after another took 130 to 240 us per restart cycle)
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    for (int i = lane; i < k; i += 32) y[i] = P.g[i];
+    __syncwarp();
+    for (int c1 = k; c1 > 0; c1 -= 32) {
+      const int c0 = c1 > 32 ? c1 - 32 : 0, row = c0 + lane;
+      // the diagonal block: lane holds row c0 + lane
+      double2 v = row < c1 ? y[row] : make_double2(0, 0);
+      for (int i = c1 - 1; i >= c0; --i) {
+        const double2 hi = row <= i ? P.H[row * ld + i] : make_double2(0, 0);
+        const double den = zabs2(hi);   // lane i - c0 holds the diagonal entry
+        double2 x = den > 0.0 ? zscale(1.0 / den, zmul(v, zconj(hi))) : make_double2(0, 0);
+        x.x = __shfl_sync(0xffffffffu, x.x, i - c0);
+        x.y = __shfl_sync(0xffffffffu, x.y, i - c0);
+        if (row == i) y[i] = x;
+        else if (row < i) v = zsub(v, zmul(hi, x));
+      }
+      __syncwarp();
+      // the rows above
+      for (int r = lane; r < c0; r += 32) {
+        double2 t = y[r];
+#pragma unroll 8
+        for (int i = c1 - 1; i >= c0; --i) t = zsub(t, zmul(P.H[r * ld + i], y[i]));
+        y[r] = t;
+      }
+      __syncwarp();
     }
   }
   __syncthreads();
@@ -182,6 +203,7 @@ __global__ void gmres_update(ArnoldiProblem* __restrict__ probs, int nprob, int 
   const double2* basis = P.Z ? P.Z : P.V;   // flexible GMRES: x += Z y
   for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
     double2 acc = P.x[r];
+#pragma unroll 8
     for (int i = 0; i < k; ++i) acc = zadd(acc, zmul(basis[(size_t)i * P.ldv + r], y[i]));
     P.x[r] = acc;
   }

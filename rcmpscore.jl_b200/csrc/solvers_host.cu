@@ -67,8 +67,9 @@ static cudaError_t gmres_cycle_launches(ArnoldiProblem* d_probs, int NP, int dp,
       if (e) break;
     }
     e = lindblad_arnoldi_launch(dp, d_probs, NP, j, stream);
-    if (!e) e = gram_schmidt_launch(d_probs, NP, j, nvec, sms, sms, stream);
-    if (!e) e = gmres_givens_launch(d_probs, NP, j, stream);
+    bool rotated = false;
+    if (!e) e = gram_schmidt_launch(d_probs, NP, j, nvec, sms, sms, stream, &rotated);
+    if (!e && !rotated) e = gmres_givens_launch(d_probs, NP, j, stream);
   }
   return e;
 }
