@@ -34,7 +34,10 @@ import numpy as np  # noqa: E402
 METRIC = "fg_phi4 evals/s at D=64 (energy + finished gradient), FP64"
 METRIC_SPLIT = ("fg_phi4 evals/s at D=64 (energy + finished gradient), split-precision trajectory products "
                 "(BF16 slices on tcgen05) vs FP64, |dE/E|<=1e-10")
-FLOPS_PER_RHS_D3 = 224      # 28 complex D^3 products (8 flops per complex multiply-add) per right-hand side
+# real flops of one quartic right-hand side over D^3: every channel is Hermitian, so each of the seven
+# needs Q X and R X in full and one triangle of (R X) R^dag, 8 flops per complex multiply-add
+FLOPS_PER_RHS_D3 = 7 * 8 * 2.5
+DENSE_FLOPS_PER_RHS_D3 = 7 * 8 * 4   # the four full products per channel of the row-block kernels
 # BF16 tensor flops the split engine executes per right-hand side of one D = 64 state (4 CTAs):
 # per CTA and chunk 28 slice pairs x 2 MMAs of M = 64, K = 16 and N = N_cat; chunks: 7 G1 units x 4
 # (N_cat 64), 3 paired G2 units x 8 (N_cat 64), 1 single G2 unit x 8 (N_cat 32)
@@ -154,7 +157,8 @@ def single_state_latency(steps):
             "phases_ms_last_call": {"trajectory": t[0], "pullback": t[1], "kinetic": t[2], "boundary_finish": t[3],
                                     "whole_call": t[4], "boundary_prepare_beside_trajectory": t[5],
                                     "boundary_gmres": t[6]},
-            "trajectory_ctas_per_state": 4 * groups.value, "channel_groups": groups.value,
+            # 4 stands for one team of CTAs per channel (7 x 16), 1 for one team per state
+            "trajectory_ctas_per_state": 16 * (7 if groups.value == 4 else 1), "channel_groups": groups.value,
             "rhs_calls": st["rhs_calls"], "accepted": st["accepted"], "rejected": st["rejected"], "energy": e}
 
 
@@ -305,7 +309,7 @@ def run_b200(args, rank, world, local_rank):
         # the split engine runs on the BF16 tensor pipe: executed BF16 flops against the measured
         # sustained cuBLAS BF16 throughput (the kernel runs inside a long step)
         bf16 = sum(SPLIT_FLOPS_PER_RHS * rhs[i] for i in range(n) if dims[i] == 64)
-        fp64eq = sum(FLOPS_PER_RHS_D3 * rhs[i] * dims[i] ** 3 * (0.25 if packed[i] else 1.0) for i in range(n))
+        fp64eq = sum(DENSE_FLOPS_PER_RHS_D3 * rhs[i] * dims[i] ** 3 * (0.25 if packed[i] else 1.0) for i in range(n))
         peaks = {}
         pf = ROOT / "MEASURED_PEAKS.json"
         if pf.exists():
@@ -324,24 +328,16 @@ def run_b200(args, rank, world, local_rank):
                 "fp64_equivalent_tflops": fp64eq / (traj_ms_split / 1000.0) / 1e12}
 
     split_roofline = split_roofline_of(traj, rhs_calls) if split else None
-    # DRAM traffic of one launch: bytes per right-hand side of one state times this launch's
-    # right-hand sides. The rate comes from an ncu capture of this very launch where one was taken
-    # (the default 32-state workload and layout: its stage vectors exceed L2 and are re-read from
-    # DRAM), otherwise from a two-state capture at the same D, a lower bound for larger batches.
+    # DRAM traffic of one launch: bytes per right-hand side of one state, from an ncu capture of this
+    # very launch (the default 32-state workload and layout), times this launch's right-hand sides
     traffic = None
     tf = ROOT / "profiles" / "trajectory_traffic.json"
     if tf.exists():
         try:
-            rec = json.loads(tf.read_text())
-            full = rec.get("measured_launches", {}).get(args.workload)
-            default_layout = (not split and args.trajectory_groups == 0 and args.quartic_route == "auto"
-                              and args.half_window == 30.0 and args.n_quad == 512 and not quartic_only)
-            if full and default_layout:
+            full = json.loads(tf.read_text()).get("measured_launches", {}).get(args.workload)
+            if (full and not split and args.trajectory_groups == 0 and args.quartic_route == "auto"
+                    and args.half_window == 30.0 and args.n_quad == 512 and not quartic_only):
                 traffic = full["dram_bytes_per_state_rhs"] * sum(rhs_calls[i] for i in range(n))
-            else:
-                per = rec.get("dram_bytes_per_state_rhs", {})
-                if all(str(d) in per for d in dims):
-                    traffic = sum(per[str(dims[i])] * rhs_calls[i] for i in range(n))
         except (OSError, ValueError, KeyError):
             traffic = None
 
@@ -485,7 +481,8 @@ def run_b200(args, rank, world, local_rank):
                                              "unpacked channels for every state")},
                 "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                              "frac": achieved / peak if peak else None, "traffic": traffic,
-                             "kernel": "trajectory_kernel<64> (FP64 mma.sync m16n8k8)",
+                             "kernel": ("trajectory_kernel" if args.trajectory_groups else
+                                        "wide_kernel or tile_kernel") + " (FP64 mma.sync m16n8k8)",
                              "peak_source": "FP64 mma.sync throughput measured in this run (rcmps_fp64_peak_tflops)",
                              "flops_per_launch": flops, "launch_ms": traj},
                 "phases_ms": {"trajectory": traj, "pullback": statistics.mean(pull_ms),

@@ -66,12 +66,14 @@ typedef struct rcmps_settings {
                                   column scales per term) for the states of padded dimension 64, FP64
                                   for the others. The DOP853 error estimate and step control, the
                                   stage sums and every solve stay FP64. */
-  int trajectory_groups;       /* FP64 quartic trajectory: CTAs per 16-row block of a state, each for
-                                  a group of channels (1, 2 or 4; a state's cluster has dp/16 times
-                                  as many CTAs, at most 16). 0 (default): the most that keeps every
-                                  state of the launch resident at once, so a lone state spreads over
-                                  up to 16 SMs and a full batch keeps one CTA per row block. Results
-                                  agree to rounding (the reductions' summation order changes). */
+  int trajectory_groups;       /* FP64 quartic trajectory. 0 (default): states whose density is Hermitian
+                                  to rounding run on Hermitian tiles, a lone state (or a few, a launch
+                                  after another) on one team of CTAs per channel, a batch on one team
+                                  per state; the layouts give the same bits. 1, 2 or 4 force the
+                                  row-block kernel (the one that states with another density take):
+                                  CTAs per 16-row block of a state, each for a group of channels (a
+                                  state's cluster has dp/16 times as many CTAs, at most 16); results
+                                  agree to rounding. */
   int boundary_preconditioner; /* boundary Poisson GMRES: 1 (default) right-preconditioned by the
                                   no-jump inverse with the Sherman-Morrison correction, as the
                                   reference solves it (numerics.py:37-71, 103-117), restart
@@ -323,7 +325,7 @@ int rcmps_lbfgs_direction(rcmps_context* context, int d, int m, const double* rh
 int rcmps_retract(rcmps_context* context, int d, const double* R, const double* K, const double* direction,
                   double alpha, double* R_out, double* K_out, void* stream);
 
-/* The tile choice of the FP64 trajectory kernel's autotuner for (system: 0 quartic, 1 all-ODE,
+/* The tile choice of the row-block FP64 trajectory kernel's autotuner for (system: 0 quartic, 1 all-ODE,
  * 2 <phi>; padded dimension dp) at the channel-group count of the last launch of that pair: the
  * depth of the operand ring (2, 3 or 4 staged chunks; 0 while not yet decided). The quartic
  * system tunes on the caller's own launches: the first three of a pair and group count take the
@@ -333,10 +335,10 @@ int rcmps_retract(rcmps_context* context, int d, const double* R, const double* 
  * route at dp 128). The depth changes the schedule only; results are identical. No counterpart
  * in the reference (its tiles follow a fixed rule, runtime/generic_layout.py:21-52). */
 int rcmps_trajectory_tuning(const rcmps_context* context, int system, int dp, int* ring, float* ms);
-/* The channel groups of the last trajectory launch of (system, dp) in this context (1, 2 or 4
- * CTAs per 16-row block of a state, rcmps_settings.trajectory_groups; 0: no launch yet). No
- * counterpart in the reference (its cooperative grid takes a fixed CTA count per state,
- * persistent_trajectory_backend.py:207-283). */
+/* The layout of the last trajectory launch of (system, dp) in this context. Row-block kernels: CTAs
+ * per 16-row block of a state (1, 2 or 4; the all-ODE system also 8 and 14). Hermitian tiles: 4 for
+ * one team per channel, 1 for one team per state. 0: no launch yet. No counterpart in the reference
+ * (its cooperative grid takes a fixed CTA count per state, persistent_trajectory_backend.py:207-283). */
 int rcmps_trajectory_groups(const rcmps_context* context, int system, int dp, int* groups);
 
 /* Number of kernel launches this library has issued in the process (all contexts). No

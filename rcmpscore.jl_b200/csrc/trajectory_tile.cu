@@ -22,15 +22,20 @@
 // coalesced 512-byte load per warp, straight into registers: no staging buffer, no copy barrier.
 // Two cluster barriers per right-hand side (X_c complete, P_c and Y_c complete).
 //
+// Measured on one B200, a lone random state, per right-hand side, row-block kernel and this one: D = 8
+// 10.3 and 2.4 us, D = 32 18.6 and 4.4, D = 64 31.4 and 5.3, Z2 D = 128 161 and 16. At D = 64: MMAs 1.9 us
+// (their floor at the DMMA peak 1.2), the two barriers 1.9, operand loads 0.6, partial tiles 0.6.
+//
 // What bounds it: the chain of dependent right-hand sides of one state. A lone state therefore takes
 // one team per channel (7 NB^2 CTAs): the insertion's P_s comes from another team through a flag per
 // tile and right-hand side, and only towards the channels that follow in the chains 0 -> 1 -> 2 and
 // 6 -> 5 -> 4 -> 3, so a team runs ahead of its followers and nobody waits inside an attempt for a
 // team behind it; the teams meet once per attempt at the error norm. Teams of one state wait for one
 // another, so such a launch is cooperative. A batch takes one team per state (wide_kernel up to
-// DP = 64) when that is faster than a few states at a time (use_teams).
+// DP = 64) when that is faster than a few states at a time (teams_for).
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <type_traits>
 #include "common.cuh"
@@ -612,7 +617,7 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
     // owned tile to shared memory between the two barriers of a right-hand side, and flags the P tile
     // after the second. Rank 0's also exchanges the records and decides on the attempt: while the
     // other warps go on with the dense stages when the step holds sample points (they are due unless
-    // the attempt is rejected, one in twenty or fewer), so the exchange, 7 to 15 us, is off the path.
+    // the attempt is rejected, a few in a hundred), so the exchange, 7 to 15 us, is off the path.
     if (warp == G::NW) {
       const int src = c_src[c0], dst = c_feeds[c0];
       const bool takes = src >= 0 && owns(c0);
@@ -1209,7 +1214,9 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
 // once per channel. The columns j of every X_c, and later the rows i of the owned P_c, land in shared
 // memory by one bulk copy per channel (they are contiguous in fragment order). A warp sums its K slices
 // in the order in which tile_kernel's warps meet, and keeps the same partial sums of the error norm:
-// the two kernels give the same bits.
+// the two kernels give the same bits. 32 x D = 64 (16 of them Z2): 24 us per right-hand side of a random
+// state on 16 CTAs, 8 states at once, against 119 us on 4 CTAs in the row-block kernel with 32 at once;
+// bound by the MMAs (13.5 of the 24 us; 9.4 at the DMMA peak) and the stage vectors' L2 traffic.
 template <int DP>
 struct Wide {
   using G = TG<DP>;
@@ -1713,20 +1720,35 @@ static int resident_clusters(K kern, int threads, size_t smem) {
   return n;
 }
 
+// The current device's capacity, a constant of device and kernel: asked once.
+template <class F>
+static int per_device(std::atomic<int> (&known)[64], F ask) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ask();
+  int n = known[dev].load();
+  if (n == 0) known[dev].store(n = ask() + 1);
+  return n - 1;
+}
 // States whose seven teams are resident at once, and those of the one-team kernel.
 template <int DP>
 static int lone_states() {
   static_assert(Smem<DP, true>::bytes() <= 232448, "shared memory per CTA");
-  return resident_clusters<DP>(tile_kernel<DP, true>, Smem<DP, true>::THREADS, Smem<DP, true>::bytes()) / kChannels;
+  static std::atomic<int> known[64];
+  return per_device(known, [] {
+    return resident_clusters<DP>(tile_kernel<DP, true>, Smem<DP, true>::THREADS, Smem<DP, true>::bytes()) / kChannels;
+  });
 }
 template <int DP>
 static int batch_states() {
-  if constexpr (TG<DP>::B == 16) {
-    return resident_clusters<DP>(wide_kernel<DP>, Wide<DP>::NT, Wide<DP>::BYTES);
-  } else {
-    static_assert(Smem<DP, false>::bytes() <= 232448, "shared memory per CTA");
-    return resident_clusters<DP>(tile_kernel<DP, false>, TG<DP>::NT, Smem<DP, false>::bytes());
-  }
+  static std::atomic<int> known[64];
+  return per_device(known, [] {
+    if constexpr (TG<DP>::B == 16) {
+      return resident_clusters<DP>(wide_kernel<DP>, Wide<DP>::NT, Wide<DP>::BYTES);
+    } else {
+      static_assert(Smem<DP, false>::bytes() <= 232448, "shared memory per CTA");
+      return resident_clusters<DP>(tile_kernel<DP, false>, TG<DP>::NT, Smem<DP, false>::bytes());
+    }
+  });
 }
 
 // Seven teams per state, a few states per launch one launch after another, or one team per state, as

@@ -81,3 +81,17 @@ def test_density_that_is_not_hermitian_takes_the_general_equations(gpu_context):
         assert got[3:] == want[3:]
         assert abs(got[0] - want[0]) <= 1e-13 * abs(want[0])
         assert np.linalg.norm(got[1] - want[1]) <= 1e-12 * np.linalg.norm(want[1])
+
+
+@pytest.mark.parametrize("d", [20, 50])
+def test_ode_channel_groups(gpu_context, d):
+    """The 26-channel system over 8 (dp 32) and 4 (dp 64) channel groups against the oracle."""
+    from rcmps_b200 import objective
+    r, k, rho = _state(d, False, 70 + d)
+    q = O.left_canonical_q(r, k)
+    got = objective.evaluate_phi4(r, q, rho, 1.5, half_window=0.5, n_quad=8)
+    ref = O.evaluate_phi4(r, q, rho, 1.5, half_window=0.5, n_quad=8)
+    assert (got["stats"]["accepted"], got["stats"]["rejected"]) == (ref["stats"]["accepted"], ref["stats"]["rejected"])
+    assert abs(got["value"] - ref["value"]) <= 1e-10 * max(1.0, abs(ref["value"]))
+    for name in ("covector", "environment"):
+        assert np.linalg.norm(got[name] - ref[name]) <= 1e-10 * max(1.0, np.linalg.norm(ref[name]))
