@@ -68,9 +68,17 @@ int kinetic_run(rcmps_context* ctx, KineticJob& job, cudaStream_t stream) {
   std::map<int, std::vector<int>> groups;
   for (int i = 0; i < job.n; ++i) groups[padded_dim(job.dims[i])].push_back(i);
   rcmps_slot& SL = ctx->slot[job.slot];
-  size_t free_b = 0, total_b = 0;
-  cudaMemGetInfo(&free_b, &total_b);
-  const size_t budget = std::max<size_t>((size_t)1 << 30, (free_b + SL.arena_bytes) * job.memory_share);
+  // asked for only when a group of states needs more than the floor (as in quartic_run)
+  const size_t memory_floor = std::max<size_t>((size_t)1 << 30, SL.arena_bytes * job.memory_share);
+  size_t budget = 0;
+  auto memory_budget = [&] {
+    if (!budget) {
+      size_t free_b = 0, total_b = 0;
+      cudaMemGetInfo(&free_b, &total_b);
+      budget = std::max<size_t>((size_t)1 << 30, (free_b + SL.arena_bytes) * job.memory_share);
+    }
+    return budget;
+  };
   cudaEventRecord(SL.ev[0], stream);
   const size_t scratch_budget = (size_t)1 << 30;
 
@@ -81,7 +89,9 @@ int kinetic_run(rcmps_context* ctx, KineticJob& job, cudaStream_t stream) {
     for (int i : all) dmax = std::max(dmax, job.dims[i]);
     const int kmax = std::min(S.krylov_maxdim, dmax * dmax);
     const size_t per = kinetic_state_bytes(dp, kmax, nshift);
-    const int cap = (int)std::max<size_t>(1, (budget - std::min(budget, scratch_budget)) / per);
+    int cap = (int)all.size();
+    if (all.size() > 1 && per * all.size() + scratch_budget > memory_floor)
+      cap = (int)std::max<size_t>(1, (memory_budget() - std::min(memory_budget(), scratch_budget)) / per);
     for (size_t start = 0; start < all.size(); start += cap) {
       const int n = (int)std::min<size_t>(cap, all.size() - start);
       const std::vector<int> idx(all.begin() + start, all.begin() + start + n);
