@@ -204,7 +204,7 @@ lindblad_kernel(const LindbladTask* __restrict__ tasks, const ArnoldiProblem* __
 //   out = [A1_i | X_i] [X_j; A1h_j] + P_i A2h_j,  P_ij = A2_i X_j.
 // Bound by latency (a GMRES step waits for one action), so it takes NB times the SMs of the row-block
 // form, splits K over the warps, reads every fragment straight from L2 and exchanges the P tiles
-// through distributed shared memory: one problem at D = 64 24.5 -> 9 us.
+// through distributed shared memory: one problem at D = 64 24.5 -> 12.6 us, at D <= 16 11.2 -> 7.3 us.
 template <int DP>
 struct LTile {
   static constexpr int B = DP <= 64 ? 16 : 32, NB = DP / B, NR = NB * NB;
@@ -560,8 +560,8 @@ inline int cgs_cluster(int n, int j, int nprob, int max_ctas) {
 
 // The new column of a GMRES problem's Hessenberg matrix: the earlier rotations, the new one, the rotated
 // residual and the stop test (gmres_givens, by one thread), on the column hc and the rotations in shared
-// memory. In the Gram-Schmidt launch it costs 2 us; as a launch of its own, one thread reading column and
-// rotations from global memory took 7 us and a launch gap.
+// memory. As a launch of its own, one thread reading column and rotations from global memory, it took
+// 7 us and a launch gap per GMRES step.
 __device__ void gmres_rotate(ArnoldiProblem& P, int j, const double2* hc, const double2* cs, const double2* sn,
                              double beta) {
   const int ld = P.kmax;
