@@ -134,7 +134,6 @@ def single_state_latency(steps):
     public single-state call (rcmps_b200.objective.objective, host arrays in and out), the call an
     L-BFGS trial makes: wall time per call after one untimed call, the device phases of the last
     call, and the trajectory's layout (CTAs per state)."""
-    import ctypes as C
     from rcmps_b200 import objective
     from rcmps_b200.batch import random_state
     R, K = random_state(64, 0)
@@ -149,16 +148,14 @@ def single_state_latency(steps):
         walls.append(time.perf_counter() - t0)
     ctx = objective.context()
     t = ctx.timings()
-    groups = C.c_int(0)
-    ctx.lib.rcmps_trajectory_groups(ctx.handle, 0, 64, C.byref(groups))
+    teams = ctx.trajectory_layout(64)[0]
     return {"workload": "1 random state D=64 (seed 0, scaling 0.2), g=2, the benchmark's settings",
             "api": "rcmps_b200.objective.objective (host arrays in and out)", "steps": steps,
             "ms_per_eval": 1000 * statistics.mean(walls), "ms_min": 1000 * min(walls),
             "phases_ms_last_call": {"trajectory": t[0], "pullback": t[1], "kinetic": t[2], "boundary_finish": t[3],
                                     "whole_call": t[4], "boundary_prepare_beside_trajectory": t[5],
                                     "boundary_gmres": t[6]},
-            # 4 stands for one team of CTAs per channel (7 x 16), 1 for one team per state
-            "trajectory_ctas_per_state": 16 * (7 if groups.value == 4 else 1), "channel_groups": groups.value,
+            "trajectory_ctas_per_state": 16 * teams, "teams_per_state": teams,
             "rhs_calls": st["rhs_calls"], "accepted": st["accepted"], "rejected": st["rejected"], "energy": e}
 
 

@@ -337,9 +337,15 @@ int rcmps_retract(rcmps_context* context, int d, const double* R, const double* 
 int rcmps_trajectory_tuning(const rcmps_context* context, int system, int dp, int* ring, float* ms);
 /* The layout of the last trajectory launch of (system, dp) in this context. Row-block kernels: CTAs
  * per 16-row block of a state (1, 2 or 4; the all-ODE system also 8 and 14). Hermitian tiles: 4 for
- * one team per channel, 1 for one team per state. 0: no launch yet. No counterpart in the reference
- * (its cooperative grid takes a fixed CTA count per state, persistent_trajectory_backend.py:207-283). */
+ * one team per channel, 1 for one team per state (rcmps_trajectory_layout tells the kernels apart).
+ * 0: no launch yet. No counterpart in the reference (its cooperative grid takes a fixed CTA count
+ * per state, persistent_trajectory_backend.py:207-283). */
 int rcmps_trajectory_groups(const rcmps_context* context, int system, int dp, int* groups);
+/* Which kernels the last quartic call of this context ran for its states of padded dimension dp:
+ * tile_states of them on Hermitian tiles, with `teams` teams of CTAs per state (7: one per channel,
+ * 1: one for all channels, 0: no state on tiles), and row_states on the row-block kernel (a density
+ * not Hermitian to 8 eps max|rho|, a forced layout, split precision). No counterpart in the reference. */
+int rcmps_trajectory_layout(const rcmps_context* context, int dp, int* teams, int* tile_states, int* row_states);
 
 /* Number of kernel launches this library has issued in the process (all contexts). No
  * counterpart in the reference. */

@@ -905,6 +905,19 @@ int rcmps_trajectory_groups(const rcmps_context* ctx, int system, int dp, int* g
   return RCMPS_INVALID_ARGUMENT;
 }
 
+int rcmps_trajectory_layout(const rcmps_context* ctx, int dp, int* teams, int* tile_states, int* row_states) {
+  if (!ctx || !teams || !tile_states || !row_states) return RCMPS_INVALID_ARGUMENT;
+  const int dps[6] = {16, 32, 48, 64, 96, 128};
+  for (int k = 0; k < 6; ++k)
+    if (dps[k] == dp) {
+      *teams = ctx->traj_layout[k][0];
+      *tile_states = ctx->traj_layout[k][1];
+      *row_states = ctx->traj_layout[k][2];
+      return RCMPS_OK;
+    }
+  return RCMPS_INVALID_ARGUMENT;
+}
+
 double rcmps_fp64_peak_tflops(rcmps_context* ctx) {
   if (!ctx) return 0.0;
   cudaSetDevice(ctx->device);

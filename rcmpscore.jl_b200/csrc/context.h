@@ -53,6 +53,9 @@ struct rcmps_context {
   int traj_ring[3][6][3] = {};
   float traj_ring_ms[3][6][3][3] = {};
   int traj_groups[3][6] = {};
+  // the last quartic call by padded dimension: teams per state on Hermitian tiles, states on tiles and
+  // states on row blocks
+  int traj_layout[6][3] = {};
 };
 
 namespace rcmps {

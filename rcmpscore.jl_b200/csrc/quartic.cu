@@ -211,6 +211,8 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
     const SysSizes zs = sys_sizes(system, dp, nblk);
     const int NCH = zs.nch;
     const size_t fixed = (size_t)(npoints + 3 * nodes) * 8 + 4096;
+    int* layout = ctx->traj_layout[dp_index(dp)];
+    if (system == 0) layout[0] = layout[1] = layout[2] = 0;
     int cap = (int)all.size();
     if (all.size() > 1 && per * all.size() + fixed > memory_floor)
       cap = (int)std::max<size_t>(1, (memory_budget() - std::min(memory_budget(), fixed)) / per);
@@ -389,6 +391,11 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
       const bool rows = nherm < n;   // states for the row-block kernel
       if (rows) tc.groups = trajectory_groups(system, dp, n, S.trajectory_groups, split ? 1 : 0);
       ctx->traj_groups[system][dp_index(dp)] = rows ? tc.groups : std::min(teams, 4);
+      if (system == 0) {
+        if (nherm) layout[0] = teams;
+        layout[1] += nherm;
+        layout[2] += n - nherm;
+      }
       if (rows && !split) tc.ring = ring_for_launch(ctx, system, dp, group_level(tc.groups));
       if (e == cudaSuccess) e = cudaEventRecord(e0, stream);
       // Teams of one state wait for one another, so only one launch of several teams is in flight on a

@@ -107,6 +107,7 @@ SIGNATURES = {
     "rcmps_retract": (_I, [_P, _I, _P, _P, _P, _D, _P, _P, _P]),
     "rcmps_trajectory_tuning": (_I, [_P, _I, _I, C.POINTER(_I), C.POINTER(C.c_float)]),
     "rcmps_trajectory_groups": (_I, [_P, _I, _I, C.POINTER(_I)]),
+    "rcmps_trajectory_layout": (_I, [_P, _I, C.POINTER(_I), C.POINTER(_I), C.POINTER(_I)]),
     "rcmps_fp64_peak_tflops": (_D, [_P]),
     "rcmps_launch_count": (C.c_longlong, []),
 }
@@ -164,6 +165,14 @@ class Context:
         buf = (C.c_float * 8)()
         self.lib.rcmps_last_timings(self.handle, buf, 8)
         return list(buf)
+
+    def trajectory_layout(self, d):
+        """(teams, tile_states, row_states) of the last quartic call's states whose bond dimension
+        pads to that of d (rcmps_trajectory_layout)."""
+        dp = next(p for p in (16, 32, 48, 64, 96, 128) if d <= p)
+        out = (C.c_int(0), C.c_int(0), C.c_int(0))
+        self.lib.rcmps_trajectory_layout(self.handle, dp, *(C.byref(x) for x in out))
+        return tuple(x.value for x in out)
 
     def close(self):
         if self.handle:

@@ -83,6 +83,21 @@ def test_density_that_is_not_hermitian_takes_the_general_equations(gpu_context):
         assert np.linalg.norm(got[1] - want[1]) <= 1e-12 * np.linalg.norm(want[1])
 
 
+@pytest.mark.parametrize("d,z2", [(12, False), (40, True)])
+def test_the_layout_tells_which_kernel_ran(gpu_context, d, z2):
+    state = _state(d, z2, 7)
+    _batch([state])
+    assert gpu_context.trajectory_layout(d) == (7, 1, 0)
+    _batch([state], groups=2)
+    assert gpu_context.trajectory_layout(d) == (0, 0, 1)
+    r, k, rho = state
+    bent = rho + 1e-9 * (r - r.conj().T)
+    _batch([(r, k, bent)], symmetry=0)
+    assert gpu_context.trajectory_layout(d) == (0, 0, 1)
+    _batch([state] * 300)
+    assert gpu_context.trajectory_layout(d) == (1, 300, 0)
+
+
 @pytest.mark.parametrize("d", [20, 50])
 def test_ode_channel_groups(gpu_context, d):
     """The 26-channel system over 8 (dp 32) and 4 (dp 64) channel groups against the oracle."""
