@@ -2,6 +2,8 @@
 with ragged and full sizes, one team per channel and one team for all channels (the same bits), the
 packed route with and without whole zero tiles, and a density that is not Hermitian (the row-block
 kernel)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -47,29 +49,66 @@ def test_quartic_against_the_oracle(gpu_context, d, z2):
         assert np.linalg.norm(g[name] - o[name]) <= 1e-11 * max(1.0, np.linalg.norm(o[name]))
 
 
+def _quartic(ctx, states, groups=0):
+    """The quartic part alone of a batch: per state the value, covector, environment and the
+    controller's record."""
+    import torch
+    from rcmps_b200 import _lib, objective
+    s = objective.settings_from_args(None, half_window=WINDOW, n_quad=NODES, symmetry=2, trajectory_groups=groups)
+    n, dims = len(states), [len(x[0]) for x in states]
+    dR, dK, dP = (objective._device(list(x)) for x in zip(*states))
+    value = torch.zeros(n, dtype=torch.float64, device="cuda")
+    cov = torch.zeros(sum(d * d for d in dims), dtype=torch.complex128, device="cuda")
+    env = torch.zeros_like(cov)
+    stats = (_lib.StateStats * n)()
+    assert ctx.lib.rcmps_quartic_batch(ctx.handle, n, (C.c_int * n)(*dims), (C.c_double * n)(*[1.0] * n), dR.data_ptr(),
+                                       dK.data_ptr(), dP.data_ptr(), C.byref(s), value.data_ptr(), cov.data_ptr(),
+                                       env.data_ptr(), stats, objective._stream()) == 0
+    cov, env = objective._unpack(cov, dims), objective._unpack(env, dims)
+    return [(value[i].item(), cov[i], env[i], stats[i].as_dict()) for i in range(n)]
+
+
+def _one_team_batch(ctx, states):
+    """The states repeated until a launch takes one team per state: (copies, results)."""
+    many = 8 * len(states)
+    while many <= 2048:
+        out = _quartic(ctx, [states[i % len(states)] for i in range(many)])
+        if ctx.trajectory_layout(len(states[0][0])) == (1, many, 0):
+            return many, out
+        many *= 2
+    raise AssertionError("no launch took one team per state")
+
+
 @pytest.mark.parametrize("d,z2", [(80, False), (96, True), (100, False), (128, True)])
 def test_large_tiles_against_the_row_blocks(gpu_context, d, z2):
     state = _state(d, z2, d)
     (e0, c0, v0, a0, r0), = _batch([state], groups=1)
-    for n in (1, 4, 20):    # a lone state, a few launches of one team per channel, one team per state
-        for e, c, v, a, r in _batch([state] * n):
+    assert gpu_context.trajectory_layout(d) == (0, 0, 1)
+    many, _ = _one_team_batch(gpu_context, [state])
+    for n, teams in ((1, 7), (4, 7), (many, 1)):
+        results = _batch([state] * n)
+        assert gpu_context.trajectory_layout(d) == (teams, n, 0)
+        for e, c, v, a, r in results:
             assert (a, r) == (a0, r0)
             assert abs(e - e0) <= 1e-12 * abs(e0)
             assert np.linalg.norm(c - c0) <= 1e-11 * np.linalg.norm(c0)
             assert np.linalg.norm(v - v0) <= 1e-11 * np.linalg.norm(v0)
 
 
-@pytest.mark.parametrize("d,many", [(9, 100), (16, 24), (24, 40), (32, 40), (40, 5), (48, 20), (50, 4), (64, 12)])
-def test_batch_and_lone_state_give_the_same_bits(gpu_context, d, many):
+@pytest.mark.parametrize("d", [9, 16, 24, 32, 40, 48, 50, 64, 80, 96, 100, 128])
+def test_batch_and_lone_state_give_the_same_bits(gpu_context, d):
     states = [_state(d, i % 2 == 1 and d % 2 == 0, 10 * d + i) for i in range(3)]
-    batch = _batch([states[i % 3] for i in range(many)])
-    for i in range(3):
-        e, c, v, a, r = _batch([states[i]])[0]
-        for j in range(i, many, 3):
-            # the kinetic part's batch sizes may round differently: the environment is the quartic's
-            assert batch[j][3:] == (a, r)
-            assert abs(batch[j][0] - e) <= 1e-13 * abs(e)
-            assert np.linalg.norm(batch[j][1] - c) <= 1e-12 * np.linalg.norm(c)
+    _, batch = _one_team_batch(gpu_context, states)
+    for i, state in enumerate(states):
+        value, cov, env, stats = _quartic(gpu_context, [state])[0]
+        assert gpu_context.trajectory_layout(d) == (7, 1, 0)
+        for b in batch[i::3]:
+            assert b[0] == value
+            assert np.array_equal(b[2], env)
+            assert np.array_equal(b[1], cov)
+            for name in ("attempts", "accepted", "rejected", "dense_steps", "t_end", "last_step", "min_step", "max_step",
+                         "packed_z2"):
+                assert b[3][name] == stats[name], name
 
 
 def test_density_that_is_not_hermitian_takes_the_general_equations(gpu_context):
