@@ -179,7 +179,8 @@ cudaError_t launch_z2_check(const double* R, const double* K, const double* rho,
   return cudaGetLastError();
 }
 
-// One CTA per state: whether rho is Hermitian to rounding. The comparison is false for a NaN.
+// One CTA per state: whether rho is Hermitian to rounding. An entry that is not finite counts as an
+// infinite deviation (fmax and the comparisons would drop a NaN), so such a density is not.
 __global__ void hermitian_check_kernel(const double2* __restrict__ rho, int dp, long long stride,
                                        int* __restrict__ flags, long long flag_stride) {
   const double2* p = rho + (long long)blockIdx.x * stride;
@@ -188,14 +189,13 @@ __global__ void hermitian_check_kernel(const double2* __restrict__ rho, int dp, 
   for (int e = threadIdx.x; e < dp * dp; e += blockDim.x) {
     const int i = e / dp, j = e % dp;
     const double2 a = p[e], b = p[j * dp + i];
-    const double d = fmax(fabs(a.x - b.x), fabs(a.y + b.y));
+    const bool finite = isfinite(a.x) && isfinite(a.y);
     top = fmax(top, fmax(fabs(a.x), fabs(a.y)));
-    off = d <= off ? off : d;   // keeps a NaN
+    off = fmax(off, finite ? fmax(fabs(a.x - b.x), fabs(a.y + b.y)) : INFINITY);
   }
   for (int o = 16; o > 0; o >>= 1) {
     top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
-    const double d = __shfl_xor_sync(0xffffffffu, off, o);
-    off = d <= off ? off : d;
+    off = fmax(off, __shfl_xor_sync(0xffffffffu, off, o));
   }
   if ((threadIdx.x & 31) == 0) {
     red[0][threadIdx.x >> 5] = top;
@@ -205,9 +205,10 @@ __global__ void hermitian_check_kernel(const double2* __restrict__ rho, int dp, 
   if (threadIdx.x == 0) {
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
       top = fmax(top, red[0][w]);
-      off = red[1][w] <= off ? off : red[1][w];
+      off = fmax(off, red[1][w]);
     }
-    flags[blockIdx.x * flag_stride] = off <= 8.0 * 2.220446049250313e-16 * top ? 1 : 0;
+    // an infinite entry makes both sides infinite
+    flags[blockIdx.x * flag_stride] = isfinite(off) && off <= 8.0 * 2.220446049250313e-16 * top ? 1 : 0;
   }
 }
 

@@ -49,21 +49,22 @@ def test_quartic_against_the_oracle(gpu_context, d, z2):
         assert np.linalg.norm(g[name] - o[name]) <= 1e-11 * max(1.0, np.linalg.norm(o[name]))
 
 
-def _quartic(ctx, states, groups=0):
+def _quartic(ctx, states, symmetry=2):
     """The quartic part alone of a batch: per state the value, covector, environment and the
     controller's record."""
     import torch
     from rcmps_b200 import _lib, objective
-    s = objective.settings_from_args(None, half_window=WINDOW, n_quad=NODES, symmetry=2, trajectory_groups=groups)
+    s = objective.settings_from_args(None, half_window=WINDOW, n_quad=NODES, symmetry=symmetry)
     n, dims = len(states), [len(x[0]) for x in states]
     dR, dK, dP = (objective._device(list(x)) for x in zip(*states))
     value = torch.zeros(n, dtype=torch.float64, device="cuda")
     cov = torch.zeros(sum(d * d for d in dims), dtype=torch.complex128, device="cuda")
     env = torch.zeros_like(cov)
     stats = (_lib.StateStats * n)()
-    assert ctx.lib.rcmps_quartic_batch(ctx.handle, n, (C.c_int * n)(*dims), (C.c_double * n)(*[1.0] * n), dR.data_ptr(),
-                                       dK.data_ptr(), dP.data_ptr(), C.byref(s), value.data_ptr(), cov.data_ptr(),
-                                       env.data_ptr(), stats, objective._stream()) == 0
+    rc = ctx.lib.rcmps_quartic_batch(ctx.handle, n, (C.c_int * n)(*dims), (C.c_double * n)(*[1.0] * n), dR.data_ptr(),
+                                     dK.data_ptr(), dP.data_ptr(), C.byref(s), value.data_ptr(), cov.data_ptr(),
+                                     env.data_ptr(), stats, objective._stream())
+    objective._raise_for(rc, ctx, stats[0], "quartic")
     cov, env = objective._unpack(cov, dims), objective._unpack(env, dims)
     return [(value[i].item(), cov[i], env[i], stats[i].as_dict()) for i in range(n)]
 
@@ -135,6 +136,20 @@ def test_the_layout_tells_which_kernel_ran(gpu_context, d, z2):
     assert gpu_context.trajectory_layout(d) == (0, 0, 1)
     _batch([state] * 300)
     assert gpu_context.trajectory_layout(d) == (1, 300, 0)
+
+
+@pytest.mark.parametrize("entry", [(0, 0), (3, 1), (1, 19), (19, 19)])
+@pytest.mark.parametrize("bad", [complex(np.nan, 0.1), complex(0.1, np.nan), complex(np.inf, 0), complex(0, -np.inf)])
+def test_a_density_that_is_not_finite_is_not_hermitian(gpu_context, entry, bad):
+    """Through the C entry (the Python calls refuse it): the general equations, which stop at once."""
+    from rcmps_b200 import objective
+    r, k, rho = _state(20, False, 5)
+    rho = rho.copy()
+    rho[entry] = bad
+    rho[entry[::-1]] = np.conj(bad)
+    with pytest.raises(objective.DeviceControlFailure, match="nonfinite_error"):
+        _quartic(gpu_context, [(r, k, rho)], symmetry=0)
+    assert gpu_context.trajectory_layout(20) == (0, 0, 1)
 
 
 @pytest.mark.parametrize("d", [20, 50])
