@@ -6,7 +6,6 @@
 #include <cmath>
 #include <cstring>
 #include <map>
-#include <mutex>
 #include <string>
 #include <vector>
 #include "../../include/rcmps_b200.h"
@@ -397,12 +396,9 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
         layout[2] += n - nherm;
       }
       if (rows && !split) tc.ring = ring_for_launch(ctx, system, dp, group_level(tc.groups));
+      TilePass pass;   // held until the trajectories end; e0 does not count the wait for it
+      if (e == cudaSuccess && nherm && teams > 1) pass.enter(ctx->device, dp, n, stream);
       if (e == cudaSuccess) e = cudaEventRecord(e0, stream);
-      // Teams of one state wait for one another, so only one launch of several teams is in flight on a
-      // device: two that share the SMs could each hold part of them and wait for the rest. Held to the
-      // end of this sub-batch; other contexts' launches of one team per state go ahead.
-      std::unique_lock<std::mutex> alone;
-      if (nherm && teams > 1) alone = std::unique_lock<std::mutex>(tile_trajectory_mutex(ctx->device));
       if (e == cudaSuccess && nherm)
         e = tile_trajectory_launch(dp, (TrajState*)P(o_states), n, (double*)P(o_points), npoints, tc, P(o_sync), teams,
                                    S.symmetry != 0, stream);
@@ -500,6 +496,7 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
         e = cudaMemcpyAsync(h_vals, P(o_vout), n * 8, cudaMemcpyDeviceToHost, stream);
       if (e == cudaSuccess) e = cudaMemcpyAsync(h_tstats, P(o_tstats), n * sizeof(TrajStats), cudaMemcpyDeviceToHost, stream);
       if (e == cudaSuccess) e = cudaMemcpyAsync(h_flag, P(o_flag), n * sizeof(int), cudaMemcpyDeviceToHost, stream);
+      if (e == cudaSuccess) pass.leave(e1);
       if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
       if (e != cudaSuccess) return fail(ctx, RCMPS_CUDA_ERROR, std::string("quartic: ") + cudaGetErrorString(e));
       float ms = 0.f;

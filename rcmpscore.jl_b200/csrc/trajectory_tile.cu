@@ -1804,9 +1804,62 @@ static cudaError_t launch(const TrajState* d_states, int nstates, const double* 
 }  // namespace tile
 
 cudaError_t tile_trajectory_init() { return dop853_upload(); }
-std::mutex& tile_trajectory_mutex(int device) {
-  static std::mutex m[64];
-  return m[device & 63];
+
+static int lone_states_for(int dp) {
+  switch (dp) {
+    case 16: return tile::lone_states<16>();
+    case 32: return tile::lone_states<32>();
+    case 48: return tile::lone_states<48>();
+    case 64: return tile::lone_states<64>();
+    case 96: return tile::lone_states<96>();
+    case 128: return tile::lone_states<128>();
+    default: return 0;
+  }
+}
+
+struct TilePass::Gate {
+  std::mutex m;
+  std::condition_variable changed;
+  int dp = 0, states = 0;               // of the launches in flight
+  unsigned long long tickets = 0, turn = 0;
+};
+TilePass::Gate& TilePass::gate(int device) {
+  static Gate gates[64];
+  return gates[device & 63];
+}
+void TilePass::enter(int device, int dp, int nstates, cudaStream_t stream) {
+  const int capacity = lone_states_for(dp), take = std::min(nstates, capacity);   // the rest in later rounds
+  Gate& g = gate(device);
+  std::unique_lock<std::mutex> lock(g.m);
+  const unsigned long long ticket = g.tickets++;
+  g.changed.wait(lock, [&] {
+    return ticket == g.turn && (g.states == 0 || (g.dp == dp && g.states + take <= capacity));
+  });
+  ++g.turn;
+  g.dp = dp;
+  g.states += take;
+  g.changed.notify_all();
+  gate_ = &g;
+  states_ = take;
+  stream_ = stream;
+}
+void TilePass::give_back() {
+  {
+    std::lock_guard<std::mutex> lock(gate_->m);
+    gate_->states -= states_;
+  }
+  gate_->changed.notify_all();
+  gate_ = nullptr;
+}
+void TilePass::leave(cudaEvent_t done) {
+  if (!gate_) return;
+  cudaEventSynchronize(done);
+  give_back();
+}
+TilePass::~TilePass() {
+  if (!gate_) return;
+  cudaStreamSynchronize(stream_);
+  give_back();
 }
 size_t tile_sync_bytes() { return sizeof(tile::Sync); }
 

@@ -3,6 +3,8 @@ with ragged and full sizes, one team per channel and one team for all channels (
 packed route with and without whole zero tiles, and a density that is not Hermitian (the row-block
 kernel)."""
 import ctypes as C
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -49,12 +51,12 @@ def test_quartic_against_the_oracle(gpu_context, d, z2):
         assert np.linalg.norm(g[name] - o[name]) <= 1e-11 * max(1.0, np.linalg.norm(o[name]))
 
 
-def _quartic(ctx, states, symmetry=2):
+def _quartic(ctx, states, symmetry=2, window=WINDOW):
     """The quartic part alone of a batch: per state the value, covector, environment and the
     controller's record."""
     import torch
     from rcmps_b200 import _lib, objective
-    s = objective.settings_from_args(None, half_window=WINDOW, n_quad=NODES, symmetry=symmetry)
+    s = objective.settings_from_args(None, half_window=window, n_quad=NODES, symmetry=symmetry)
     n, dims = len(states), [len(x[0]) for x in states]
     dR, dK, dP = (objective._device(list(x)) for x in zip(*states))
     value = torch.zeros(n, dtype=torch.float64, device="cuda")
@@ -150,6 +152,62 @@ def test_a_density_that_is_not_finite_is_not_hermitian(gpu_context, entry, bad):
     with pytest.raises(objective.DeviceControlFailure, match="nonfinite_error"):
         _quartic(gpu_context, [(r, k, rho)], symmetry=0)
     assert gpu_context.trajectory_layout(20) == (0, 0, 1)
+
+
+def _in_threads(jobs):
+    """The jobs side by side, a host thread and a stream each: their results and the wall time."""
+    import torch
+    out, start = [None] * len(jobs), threading.Barrier(len(jobs) + 1)
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            start.wait()
+            out[i] = jobs[i]()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for t in threads:
+        t.start()
+    start.wait()
+    t0 = time.perf_counter()
+    for t in threads:
+        t.join()
+    return out, time.perf_counter() - t0
+
+
+def test_lone_states_of_several_contexts_run_side_by_side(gpu_context):
+    """Four contexts with a D = 32 state each (28 CTAs): the device holds all four at once, so four
+    threads take far less than four times the time of one; and no call's trajectory time holds another's."""
+    from rcmps_b200 import _lib
+    state = _state(32, False, 3)
+    contexts = [_lib.Context(0) for _ in range(4)]
+
+    def job(ctx):
+        return lambda: [(_quartic(ctx, [state], window=30.0)[0][:3], ctx.timings()[0]) for _ in range(6)]
+    for ctx in contexts:
+        job(ctx)()
+    alone, t1 = _in_threads([job(contexts[0])])
+    together, t4 = _in_threads([job(ctx) for ctx in contexts])
+    want = alone[0][0][0]
+    for calls in together:
+        for got, _ in calls:
+            assert got[0] == want[0] and np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2])
+    assert t4 < 2.5 * t1
+    assert np.median([ms for calls in together for _, ms in calls]) < 2.0 * np.median([ms for _, ms in alone[0]])
+
+
+def test_contexts_with_states_of_several_sizes(gpu_context):
+    """Lone states, a few states per launch and one team per state from six contexts at once: the
+    bits of each alone."""
+    from rcmps_b200 import _lib
+    work = [[_state(d, i % 2 == 1, 90 + i) for i in range(n)] for d, n in
+            ((16, 1), (16, 40), (64, 1), (64, 3), (96, 1), (32, 2))]
+    contexts = [_lib.Context(0) for _ in work]
+    want = [_quartic(ctx, states) for ctx, states in zip(contexts, work)]
+    jobs = [lambda ctx=ctx, states=states: [_quartic(ctx, states) for _ in range(5)]
+            for ctx, states in zip(contexts, work)]
+    for calls, ref in zip(_in_threads(jobs)[0], want):
+        for got in calls:
+            for g, w in zip(got, ref):
+                assert g[0] == w[0] and np.array_equal(g[1], w[1]) and np.array_equal(g[2], w[2])
 
 
 @pytest.mark.parametrize("d", [20, 50])
