@@ -70,7 +70,9 @@ typedef struct rcmps_settings {
                                   to rounding run on Hermitian tiles, a lone state (or a few, a launch
                                   after another) on one team of CTAs per channel, a batch on one team
                                   per state; the layouts give the same bits. 1, 2 or 4 force the
-                                  row-block kernel (the one that states with another density take):
+                                  row-block kernel (the one that states with another density take,
+                                  and with them the Hermitian ones of the same padded dimension
+                                  while the launch holds them all at once):
                                   CTAs per 16-row block of a state, each for a group of channels (a
                                   state's cluster has dp/16 times as many CTAs, at most 16); results
                                   agree to rounding. */
@@ -344,7 +346,7 @@ int rcmps_trajectory_groups(const rcmps_context* context, int system, int dp, in
 /* Which kernels the last quartic call of this context ran for its states of padded dimension dp:
  * tile_states of them on Hermitian tiles, with `teams` teams of CTAs per state (7: one per channel,
  * 1: one for all channels, 0: no state on tiles), and row_states on the row-block kernel (a density
- * not Hermitian to 8 eps max|rho|, a forced layout, split precision). No counterpart in the reference. */
+ * not Hermitian to 8 eps max|rho| or beside one, a forced layout, split precision). No counterpart in the reference. */
 int rcmps_trajectory_layout(const rcmps_context* context, int dp, int* teams, int* tile_states, int* row_states);
 
 /* Number of kernel launches this library has issued in the process (all contexts). No

@@ -381,6 +381,14 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
           }
         }
       }
+      // A call of both kinds: the Hermitian states go with the others unless that adds a wave to the
+      // row-block launch, which lasts as long as its longest state. Split, the two launches run one
+      // after another (one of 32 states at D = 64 not Hermitian: 1073 ms split, 676 together; one of
+      // 10 at D = 16: 40 and 34).
+      if (nherm && nherm < n) {
+        const int resident = std::max(1, trajectory_resident(dp));
+        if ((n + resident - 1) / resident <= (n - nherm + resident - 1) / resident) nherm = 0;
+      }
       if (e == cudaSuccess)
         e = node_weights_launch((double*)P(o_points), (double*)P(o_weights), nodes, (double*)P(o_wj), stream);
       TrajControls tc;
@@ -388,7 +396,7 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
       tc.initial_h = S.initial_step;
       tc.max_ns = (unsigned long long)(S.max_device_seconds * 1e9);
       const bool rows = nherm < n;   // states for the row-block kernel
-      if (rows) tc.groups = trajectory_groups(system, dp, n, S.trajectory_groups, split ? 1 : 0);
+      if (rows) tc.groups = trajectory_groups(system, dp, n - nherm, S.trajectory_groups, split ? 1 : 0);
       ctx->traj_groups[system][dp_index(dp)] = rows ? tc.groups : std::min(teams, 4);
       if (system == 0) {
         if (nherm) layout[0] = teams;

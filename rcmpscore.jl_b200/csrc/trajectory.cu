@@ -1129,6 +1129,20 @@ static cudaError_t prepare_kernel() {
   return e;
 }
 
+// Clusters of G x cg CTAs the device holds at once (0 when it cannot place one).
+template <int DP, int SYS, int ENG>
+static int resident_clusters(int cg) {
+  if (prepare_kernel<DP, SYS, ENG>() != cudaSuccess) return 0;
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = launch_config<DP, SYS, ENG>(1, Geo<DP, SYS>::G * cg, nullptr, attr);
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, trajectory_kernel<DP, SYS, ENG>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return clusters;
+}
+
 // Channel groups for nstates states (see trajectory_groups).
 template <int DP, int SYS, int ENG>
 static int choose_groups(int nstates, int requested) {
@@ -1141,27 +1155,16 @@ static int choose_groups(int nstates, int requested) {
       if (counts[k] == cg) return GE::G * cg <= 16;
     return false;
   };
-  // clusters of G x cg CTAs the device holds at once (0 when it cannot place one)
-  auto resident = [&](int cg) {
-    if (prepare_kernel<DP, SYS, ENG>() != cudaSuccess) return 0;
-    cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = launch_config<DP, SYS, ENG>(nstates, GE::G * cg, nullptr, attr);
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, trajectory_kernel<DP, SYS, ENG>, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
-    return clusters;
-  };
   if (requested > 0) {   // the largest supported count up to the request
     for (int cg = requested; cg > 1; cg /= 2)
-      if (allowed(cg) && resident(cg) >= 1) return cg;
+      if (allowed(cg) && resident_clusters<DP, SYS, ENG>(cg) >= 1) return cg;
     return 1;
   }
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return 1;
   for (int k = kGroupLevels - 1; k > 0; --k)
-    if (allowed(counts[k]) && (long long)nstates * GE::G * counts[k] <= sms && resident(counts[k]) >= nstates)
+    if (allowed(counts[k]) && (long long)nstates * GE::G * counts[k] <= sms &&
+        resident_clusters<DP, SYS, ENG>(counts[k]) >= nstates)
       return counts[k];
   return 1;
 }
@@ -1468,6 +1471,18 @@ static int groups_sys(int dp, int nstates, int requested) {
     case 64: return choose_groups<64, SYS, 0>(nstates, requested);
     case 96: return choose_groups<96, SYS, 0>(nstates, requested);
     case 128: return choose_groups<128, SYS, 0>(nstates, requested);
+    default: return 0;
+  }
+}
+
+int trajectory_resident(int dp) {
+  switch (dp) {
+    case 16: return resident_clusters<16, kSysQuartic, 0>(1);
+    case 32: return resident_clusters<32, kSysQuartic, 0>(1);
+    case 48: return resident_clusters<48, kSysQuartic, 0>(1);
+    case 64: return resident_clusters<64, kSysQuartic, 0>(1);
+    case 96: return resident_clusters<96, kSysQuartic, 0>(1);
+    case 128: return resident_clusters<128, kSysQuartic, 0>(1);
     default: return 0;
   }
 }

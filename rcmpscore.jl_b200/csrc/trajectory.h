@@ -69,6 +69,7 @@ int trajectory_channels(int system);
 // that one) and 14 on the all-ODE system. A state's cluster has dp/16 x groups CTAs (at most 16). The
 // split engine and the <phi> system take 1.
 int trajectory_groups(int system, int dp, int nstates, int requested, int engine = 0);
+int trajectory_resident(int dp);   // states of the quartic system resident at once in one group
 cudaError_t node_weights_launch(const double* d_points, const double* d_weights, int n, double* d_wj,
                                 cudaStream_t stream);
 

@@ -140,6 +140,28 @@ def test_the_layout_tells_which_kernel_ran(gpu_context, d, z2):
     assert gpu_context.trajectory_layout(d) == (1, 300, 0)
 
 
+def test_states_beside_one_that_is_not_hermitian(gpu_context):
+    """Few states ride along in the row-block launch; more than it holds at once (it runs at most 16
+    CTAs per SM) take their own, and keep their bits."""
+    r, k, rho = _state(12, False, 3)
+    bent = (r, k, rho + 1e-9 * (r - r.conj().T))
+    want = _quartic(gpu_context, [(r, k, rho)], symmetry=0)[0]
+    for few in (1, 30):
+        got = _quartic(gpu_context, [bent] + [(r, k, rho)] * few, symmetry=0)
+        assert gpu_context.trajectory_layout(12) == (0, 0, few + 1)
+        for g in got[1:]:
+            assert g[3]["accepted"] == want[3]["accepted"]
+            assert abs(g[0] - want[0]) <= 1e-13 * abs(want[0])
+            assert np.linalg.norm(g[1] - want[1]) <= 1e-12 * np.linalg.norm(want[1])
+    many = 2400
+    got = _quartic(gpu_context, [bent] + [(r, k, rho)] * many, symmetry=0)
+    assert gpu_context.trajectory_layout(12) == (1, many, 1)
+    for g in got[1::100]:
+        assert g[0] == want[0] and np.array_equal(g[1], want[1]) and np.array_equal(g[2], want[2])
+    alone = _quartic(gpu_context, [bent], symmetry=0)[0]
+    assert abs(got[0][0] - alone[0]) <= 1e-13 * abs(alone[0])
+
+
 @pytest.mark.parametrize("entry", [(0, 0), (3, 1), (1, 19), (19, 19)])
 @pytest.mark.parametrize("bad", [complex(np.nan, 0.1), complex(0.1, np.nan), complex(np.inf, 0), complex(0, -np.inf)])
 def test_a_density_that_is_not_finite_is_not_hermitian(gpu_context, entry, bad):
