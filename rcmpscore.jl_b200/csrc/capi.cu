@@ -723,14 +723,16 @@ int rcmps_fg_phi4_batch_controls(rcmps_context* ctx, int n, const int* dims, con
   kj.stats = kst.data();
   kj.slot = 1;
   kj.memory_share = 0.3;
-  // SMs that the trajectories leave to the kinetic term
+  // SMs that the trajectories leave to the kinetic term, where they run on tiles (a CTA on an SM while
+  // there are SMs without one). Beside row blocks it takes what it takes alone: their few CTAs leave room
+  // for its clusters (8 states at D = 64 in one group, kinetic term 133 ms by the tiles' count, 69 so).
   int busy = 0;
   for (int dp : {16, 32, 48, 64, 96, 128}) {
     int count = 0;
     for (int i = 0; i < n; ++i) count += padded_dim(dims[i]) == dp;
-    if (count) busy = std::max(busy, tile_trajectory_ctas(dp, count));
+    if (count && quartic_on_tiles(*settings, dp)) busy = std::max(busy, tile_trajectory_ctas(dp, count));
   }
-  kj.spare_sms = std::max(16, ctx->sms - busy);
+  kj.spare_sms = busy ? std::max(16, ctx->sms - busy) : ctx->sms;
   // The kinetic term runs on its own thread and stream, the quartic term on another. The boundary
   // solve needs only the environment, which the quartic term writes right after its trajectory:
   // the solve starts then and runs while the quartic pullback produces the covector.

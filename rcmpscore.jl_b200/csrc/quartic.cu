@@ -165,6 +165,10 @@ static void ring_record(rcmps_context* ctx, int system, int dp, int level, int d
   ctx->traj_ring[system][dp_index(dp)][level] = choice;
 }
 
+bool quartic_on_tiles(const rcmps_settings& S, int dp) {
+  return S.trajectory_groups == 0 && !split_engine_for(S, 0, dp);
+}
+
 int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
   const rcmps_settings& S = job.settings;
   std::vector<double> points, weights;
@@ -354,7 +358,7 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
                             (long long)(sizeof(TrajState) / sizeof(int)), stream);
       // The tile kernel takes the states with a Hermitian density unless the caller asked for the
       // split products or for a row-block layout; the row-block kernel takes the others.
-      const bool tile_route = system == 0 && !split && S.trajectory_groups == 0;
+      const bool tile_route = system == 0 && quartic_on_tiles(S, dp);
       const int teams = tile_route ? tile_trajectory_teams(dp, n) : 0;
       if (e == cudaSuccess && teams)
         e = launch_hermitian_check(dP, dp, in_stride, n, reinterpret_cast<int*>(base + o_states + offsetof(TrajState, herm)),

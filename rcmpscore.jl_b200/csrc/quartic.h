@@ -34,6 +34,8 @@ struct QuarticJob {
 };
 
 cudaError_t quartic_init();
+// Whether the settings leave the quartic term's states of padded dimension dp to the tile kernels.
+bool quartic_on_tiles(const rcmps_settings& S, int dp);
 int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream);
 
 void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w);

@@ -114,6 +114,26 @@ def test_batch_and_lone_state_give_the_same_bits(gpu_context, d):
                 assert b[3][name] == stats[name], name
 
 
+@pytest.mark.parametrize("control", [dict(trajectory_groups=4), dict(precision=1)])
+def test_kinetic_term_beside_row_blocks_is_the_one_alone(gpu_context, control):
+    """Beside a trajectory on few CTAs the Gram-Schmidt steps keep their clusters, so the sums keep their
+    order: the kinetic value in the call has the bits of the kinetic entry's."""
+    import torch
+    from rcmps_b200 import _lib, objective
+    r, k, rho = _state(64, False, 4)
+    s = objective.settings_from_args(None, half_window=WINDOW, n_quad=NODES, kinetic_nodes=64, symmetry=0, **control)
+    _, _, stats = objective.fg_phi4_batch([r], [k], [rho], [1.0], s)
+    value = torch.zeros(1, dtype=torch.float64, device="cuda")
+    alone = (_lib.StateStats * 1)()
+    dR, dK, dP = (objective._device([x]) for x in (r, k, rho))
+    assert gpu_context.lib.rcmps_kinetic_batch(gpu_context.handle, 1, (C.c_int * 1)(64), dR.data_ptr(), dK.data_ptr(),
+                                               dP.data_ptr(), C.byref(s), value.data_ptr(), None, None, alone,
+                                               objective._stream()) == 0
+    assert stats[0]["krylov_basis"] == alone[0].as_dict()["krylov_basis"]
+    assert stats[0]["kinetic_value"] == value.item()
+    assert stats[0]["krylov_residual"] == alone[0].krylov_residual
+
+
 def test_density_that_is_not_hermitian_takes_the_general_equations(gpu_context):
     r, k, rho = _state(12, False, 3)
     bent = rho + 1e-9 * (r - r.conj().T)
