@@ -38,6 +38,7 @@
 #include <atomic>
 #include <cstdint>
 #include <type_traits>
+#include "capacity.h"
 #include "common.cuh"
 #include "dop853_device.cuh"
 #include "trajectory.h"
@@ -1706,7 +1707,7 @@ static cudaError_t configure(K kern, int nclusters, int threads, size_t smem, bo
   return e;
 }
 
-// Clusters of a kernel that the device holds at once (0: it cannot place one).
+// Clusters of a kernel that the device holds at once (0: it cannot place one; -1: the query failed).
 template <int DP, class K>
 static int resident_clusters(K kern, int threads, size_t smem) {
   cudaLaunchAttribute attr[2];
@@ -1715,19 +1716,17 @@ static int resident_clusters(K kern, int threads, size_t smem) {
   if (configure<DP>(kern, 1, threads, smem, false, nullptr, attr, cfg) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
     cudaGetLastError();
-    return 0;
+    return -1;
   }
   return n;
 }
 
-// The current device's capacity, a constant of device and kernel: asked once.
+// The current device's capacity, a constant of device and kernel.
 template <class F>
 static int per_device(std::atomic<int> (&known)[64], F ask) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ask();
-  int n = known[dev].load();
-  if (n == 0) known[dev].store(n = ask() + 1);
-  return n - 1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return std::max(0, ask());
+  return capacity_once(known[dev], ask);
 }
 // States whose seven teams are resident at once, and those of the one-team kernel.
 template <int DP>
@@ -1735,7 +1734,8 @@ static int lone_states() {
   static_assert(Smem<DP, true>::bytes() <= 232448, "shared memory per CTA");
   static std::atomic<int> known[64];
   return per_device(known, [] {
-    return resident_clusters<DP>(tile_kernel<DP, true>, Smem<DP, true>::THREADS, Smem<DP, true>::bytes()) / kChannels;
+    const int n = resident_clusters<DP>(tile_kernel<DP, true>, Smem<DP, true>::THREADS, Smem<DP, true>::bytes());
+    return n < 0 ? n : n / kChannels;
   });
 }
 template <int DP>

@@ -2,12 +2,13 @@
 quartic route chosen from the optimizer's arguments (sweep_driver.py:48-50)."""
 from __future__ import annotations
 
+import subprocess
 from types import SimpleNamespace
 
 import numpy as np
 import pytest
 
-from conftest import load_records
+from conftest import ROOT, load_records
 from oracle import fg_phi4_oracle as O
 
 
@@ -40,3 +41,28 @@ def test_validation_rows_and_refined_controls():
     assert validate.REFINED == dict(window=40.0, quadrature=1024, atol=1e-14, rtol=1e-13)
     with pytest.raises(ValueError):
         validate.source_integral(0.0)
+
+
+def _run_host_program(tmp_path, header, body):
+    """Compile and run `body` as main() against a host-only header of csrc."""
+    src = tmp_path / "main.cpp"
+    src.write_text(f'#include "{ROOT / "rcmpscore.jl_b200" / "csrc" / header}"\n#include <cstdio>\n{body}')
+    exe = tmp_path / "main"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-o", str(exe), str(src)], check=True)
+    return subprocess.run([str(exe)], capture_output=True, text=True, check=True, timeout=60).stdout.split()
+
+
+def test_a_failed_capacity_query_is_asked_again(tmp_path):
+    out = _run_host_program(tmp_path, "capacity.h", """
+int main() {
+  std::atomic<int> known{0};
+  const int answers[] = {-1, 5, 7};
+  int asked = 0;
+  auto ask = [&] { return answers[asked++]; };
+  for (int i = 0; i < 3; ++i) std::printf("%d ", rcmps::capacity_once(known, ask));
+  std::atomic<int> none{0};
+  int zeros = 0;
+  for (int i = 0; i < 2; ++i) std::printf("%d ", rcmps::capacity_once(none, [&] { ++zeros; return 0; }));
+  std::printf("%d %d", asked, zeros);
+}""")
+    assert out == ["0", "5", "5", "0", "0", "2", "1"]
