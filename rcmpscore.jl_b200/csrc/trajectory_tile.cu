@@ -1817,49 +1817,27 @@ static int lone_states_for(int dp) {
   }
 }
 
-struct TilePass::Gate {
-  std::mutex m;
-  std::condition_variable changed;
-  int dp = 0, states = 0;               // of the launches in flight
-  unsigned long long tickets = 0, turn = 0;
-};
-TilePass::Gate& TilePass::gate(int device) {
-  static Gate gates[64];
-  return gates[device & 63];
+static Admission& admission(int device) {
+  static Admission all[64];
+  return all[device & 63];
 }
 void TilePass::enter(int device, int dp, int nstates, cudaStream_t stream) {
-  const int capacity = lone_states_for(dp), take = std::min(nstates, capacity);   // the rest in later rounds
-  Gate& g = gate(device);
-  std::unique_lock<std::mutex> lock(g.m);
-  const unsigned long long ticket = g.tickets++;
-  g.changed.wait(lock, [&] {
-    return ticket == g.turn && (g.states == 0 || (g.dp == dp && g.states + take <= capacity));
-  });
-  ++g.turn;
-  g.dp = dp;
-  g.states += take;
-  g.changed.notify_all();
-  gate_ = &g;
-  states_ = take;
+  const int capacity = lone_states_for(dp);
+  states_ = std::min(nstates, capacity);   // the rest follow in later rounds
+  admission_ = &admission(device);
   stream_ = stream;
-}
-void TilePass::give_back() {
-  {
-    std::lock_guard<std::mutex> lock(gate_->m);
-    gate_->states -= states_;
-  }
-  gate_->changed.notify_all();
-  gate_ = nullptr;
+  admission_->enter(dp, states_, capacity);
 }
 void TilePass::leave(cudaEvent_t done) {
-  if (!gate_) return;
+  if (!admission_) return;
   cudaEventSynchronize(done);
-  give_back();
+  admission_->leave(states_);
+  admission_ = nullptr;
 }
 TilePass::~TilePass() {
-  if (!gate_) return;
+  if (!admission_) return;
   cudaStreamSynchronize(stream_);
-  give_back();
+  admission_->leave(states_);
 }
 size_t tile_sync_bytes() { return sizeof(tile::Sync); }
 

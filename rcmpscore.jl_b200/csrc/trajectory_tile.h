@@ -1,11 +1,11 @@
 // Host interface of the tile trajectory kernel (internal to the library).
 #pragma once
 #include <cuda_runtime.h>
-#include <condition_variable>
-#include <mutex>
 #include "trajectory.h"
 
 namespace rcmps {
+
+class Admission;   // capacity.h
 
 cudaError_t tile_trajectory_init();       // constant tables on the current device
 size_t tile_sync_bytes();                 // device bytes per state for the teams' flags and records
@@ -16,18 +16,15 @@ int tile_trajectory_ctas(int dp, int nstates);   // CTAs it keeps busy
 // Admission of launches of several teams per state to their device. Teams of one state wait for one
 // another, so every cluster of the launches in flight must be resident: two launches that share the SMs
 // could each hold part of them and wait for the rest. Launches of one padded dimension have the same
-// clusters and share the device up to the states it holds; another dimension waits until it is empty.
-// First come, first served; launches of one team per state need none.
+// clusters and share the device up to the states it holds; another dimension waits until it is empty
+// (Admission). Launches of one team per state need none.
 class TilePass {
  public:
   void enter(int device, int dp, int nstates, cudaStream_t stream);
   void leave(cudaEvent_t done);   // waits for `done`, recorded behind the launches
   ~TilePass();                    // of a call that failed: waits for the stream
  private:
-  struct Gate;
-  static Gate& gate(int device);
-  void give_back();
-  Gate* gate_ = nullptr;
+  Admission* admission_ = nullptr;
   int states_ = 0;
   cudaStream_t stream_ = nullptr;
 };

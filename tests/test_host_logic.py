@@ -66,3 +66,43 @@ int main() {
   std::printf("%d %d", asked, zeros);
 }""")
     assert out == ["0", "5", "5", "0", "0", "2", "1"]
+
+
+def test_admission_of_launches(tmp_path):
+    """One kind at a time up to its capacity, in the order of arrival."""
+    out = _run_host_program(tmp_path, "capacity.h", """
+#include <chrono>
+#include <thread>
+#include <vector>
+int main() {
+  rcmps::Admission gate;
+  std::atomic<int> inside[3] = {}, broken{0};
+  const int capacity[3] = {1, 5, 21};
+  std::vector<std::thread> threads;
+  for (int i = 0; i < 90; ++i)
+    threads.emplace_back([&, i] {
+      const int kind = i / 7 % 3, count = 1 + i % capacity[kind];
+      gate.enter(kind, count, capacity[kind]);
+      const int now = inside[kind] += count;
+      if (now > capacity[kind] || inside[(kind + 1) % 3] || inside[(kind + 2) % 3]) ++broken;
+      std::this_thread::sleep_for(std::chrono::milliseconds(2));
+      inside[kind] -= count;
+      gate.leave(count);
+    });
+  for (auto& t : threads) t.join();
+  // a later launch of the kind inside does not overtake one of another kind
+  gate.enter(2, 1, 21);
+  std::atomic<int> order{0};
+  int other = 0, same = 0;
+  auto wait = [] { std::this_thread::sleep_for(std::chrono::milliseconds(200)); };
+  std::thread a([&] { gate.enter(0, 1, 1); other = ++order; gate.leave(1); });
+  wait();
+  std::thread b([&] { gate.enter(2, 1, 21); same = ++order; gate.leave(1); });
+  wait();
+  const int early = order;
+  gate.leave(1);
+  a.join();
+  b.join();
+  std::printf("%d %d %d %d", (int)broken, early, other, same);
+}""")
+    assert out == ["0", "0", "1", "2"]
