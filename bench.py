@@ -159,6 +159,16 @@ def single_state_latency(steps):
             "rhs_calls": st["rhs_calls"], "accepted": st["accepted"], "rejected": st["rejected"], "energy": e}
 
 
+def launch_traffic(workload, rhs_calls):
+    """DRAM bytes of the trajectory launch of a workload: bytes per right-hand side of one state, from
+    an ncu capture of that launch (profiles/trajectory_traffic.json), times the launch's right-hand
+    sides; None for a workload without a capture."""
+    captures = json.loads((ROOT / "profiles" / "trajectory_traffic.json").read_text())["measured_launches"]
+    if workload not in captures:
+        return None
+    return captures[workload]["dram_bytes_per_state_rhs"] * sum(rhs_calls)
+
+
 # ----------------------------------------------------------------------------- reference arm
 def run_reference(args, rank, world):
     """The oracle (the NumPy restatement of the reference's path) on the host cores: one state per
@@ -325,18 +335,10 @@ def run_b200(args, rank, world, local_rank):
                 "fp64_equivalent_tflops": fp64eq / (traj_ms_split / 1000.0) / 1e12}
 
     split_roofline = split_roofline_of(traj, rhs_calls) if split else None
-    # DRAM traffic of one launch: bytes per right-hand side of one state, from an ncu capture of this
-    # very launch (the default 32-state workload and layout), times this launch's right-hand sides
     traffic = None
-    tf = ROOT / "profiles" / "trajectory_traffic.json"
-    if tf.exists():
-        try:
-            full = json.loads(tf.read_text()).get("measured_launches", {}).get(args.workload)
-            if (full and not split and args.trajectory_groups == 0 and args.quartic_route == "auto"
-                    and args.half_window == 30.0 and args.n_quad == 512 and not quartic_only):
-                traffic = full["dram_bytes_per_state_rhs"] * sum(rhs_calls[i] for i in range(n))
-        except (OSError, ValueError, KeyError):
-            traffic = None
+    if (not split and args.trajectory_groups == 0 and args.quartic_route == "auto" and args.half_window == 30.0
+            and args.n_quad == 512 and not quartic_only):
+        traffic = launch_traffic(args.workload, rhs_calls)
 
     # end to end through the host-buffer C entry: copies of inputs and results inside the timed region
     e2e = None

@@ -106,3 +106,11 @@ int main() {
   std::printf("%d %d %d %d", (int)broken, early, other, same);
 }""")
     assert out == ["0", "0", "1", "2"]
+
+
+def test_the_benchmark_finds_the_traffic_of_its_default_launch():
+    import bench
+    per = bench.launch_traffic("d64_mixed", [1])
+    assert 1e4 < per < 1e7
+    assert bench.launch_traffic("d64_mixed", [3, 4]) == 7 * per
+    assert bench.launch_traffic("no such workload", [1]) is None
