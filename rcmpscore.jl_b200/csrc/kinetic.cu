@@ -1197,11 +1197,10 @@ __global__ void __launch_bounds__(kSumRows* kSumGroups) contract_sum(ContractArg
   vpart = warp_sum(vpart);
   if (lane == 0) vsh[g] = vpart;
   __syncthreads();
-  const int slot[6] = {0, 1, 2, 3, 4, 5};
   if (g < 6) {
     double2 t = sh[0][g][lane];
     for (int i = 1; i < kSumGroups; ++i) t = zadd(t, sh[i][g][lane]);
-    a.fin[((size_t)s * kFinMats + 8 * op + slot[g]) * MAT + e] = t;
+    a.fin[((size_t)s * kFinMats + 8 * op + g) * MAT + e] = t;
   }
   if (threadIdx.x == 0) {
     double t = 0.0;

@@ -84,8 +84,8 @@ cudaError_t arnoldi_tasks_launch(const ArnoldiProblem* d_probs, int nprob, int j
                                 cudaStream_t s);
 cudaError_t arnoldi_start_launch(ArnoldiProblem* d_probs, int nprob, cudaStream_t s);
 cudaError_t cgs_step_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, cudaStream_t s);
-// The same Gram-Schmidt step in one launch, with the Givens step of GMRES problems (a cluster per problem, max_ctas for all of them where that
-// leaves at least one; no partial or norm arrays).
+// The same Gram-Schmidt step in one launch, with the Givens step of GMRES problems (a cluster per
+// problem, max_ctas for all of them where that leaves at least one; no partial or norm arrays).
 cudaError_t cgs_fused_launch(ArnoldiProblem* d_probs, int nprob, int j, int n, int max_ctas, cudaStream_t s);
 // The Gram-Schmidt step by whichever of the two forms suits the batch (sms: the device's SMs; spare:
 // those that work running beside this leaves free). The one-launch form also does the Givens step of

@@ -35,8 +35,8 @@ constexpr int kNodesPerBlock = 32;
 
 // Per-system sizes: channels of a stage vector, operator matrices, stage vectors of the
 // trajectory workspace (k[18], the last two of them y and prop, z[2], P, and L for the all-ODE
-// route; the quartic system's tile kernels have two partial sums behind k[18], z[3] and P[32]), pullback scratch, partial and
-// finalize matrices per state.
+// route; the quartic system's tile kernels have two partial sums behind k[18], z[3] and P[32]),
+// pullback scratch, partial and finalize matrices per state.
 struct SysSizes {
   int nch, nops, nwork;
   size_t wscr, part, fin;   // in dp x dp matrices per state
@@ -361,7 +361,8 @@ int quartic_run(rcmps_context* ctx, QuarticJob& job, cudaStream_t stream) {
       const bool tile_route = system == 0 && quartic_on_tiles(S, dp);
       const int teams = tile_route ? tile_trajectory_teams(dp, n) : 0;
       if (e == cudaSuccess && teams)
-        e = launch_hermitian_check(dP, dp, in_stride, n, reinterpret_cast<int*>(base + o_states + offsetof(TrajState, herm)),
+        e = launch_hermitian_check(dP, dp, in_stride, n,
+                                   reinterpret_cast<int*>(base + o_states + offsetof(TrajState, herm)),
                                    (long long)(sizeof(TrajState) / sizeof(int)), stream);
       int nherm = 0;
       if (e == cudaSuccess && (teams || (system == 0 && S.symmetry == 1))) {

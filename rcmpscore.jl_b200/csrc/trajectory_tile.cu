@@ -1217,7 +1217,8 @@ tile_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
 // in the order in which tile_kernel's warps meet, and keeps the same partial sums of the error norm:
 // the two kernels give the same bits. 32 x D = 64 (16 of them Z2): 24 us per right-hand side of a random
 // state on 16 CTAs, 8 states at once, against 119 us on 4 CTAs in the row-block kernel with 32 at once;
-// bound by the MMAs (13.5 of the 24 us; 9.4 at the DMMA peak) and the stage vectors' L2 traffic.
+// bound by the MMAs (13.5 of the 24 us; 9.4 at the DMMA peak) and, between them, by barriers and the stage
+// vectors' round trips to L2 (its bandwidth is at 10%; two CTAs per SM at D = 32: 17%).
 template <int DP>
 struct Wide {
   using G = TG<DP>;
@@ -1449,7 +1450,7 @@ wide_kernel(const TrajState* __restrict__ states, const double* __restrict__ poi
 
   // Stage sums and error estimates as in tile_kernel: with one column tile per warp all but the last
   // term is summed during the right-hand side before (slots 18 and 19); with two, where two CTAs share an
-  // SM and the stage vectors' L2 traffic sets the pace, when it is used.
+  // SM and the stage vectors' L2 round trips set the pace, when it is used.
   constexpr bool EARLY = NPT == 1;
   auto entry_sum = [&](const double* w, int n, double h, auto max, int e) -> double2 {
     constexpr int MAX = decltype(max)::value;
